@@ -32,6 +32,7 @@
 #include <utility>
 
 #include "hg_crmath.cuh"
+#include "hg_exact.cuh"
 #include "hg_tableaux.h"
 #include "hitengpu.h"
 
@@ -86,27 +87,31 @@ struct DopTab {
 // ---------------------------------------------------------------------------
 
 // dynamics/rtbp.py:30-74 (_crtbp_accel), numba lowering of ** (x*x, x*(x*x)).
-// The six quotients share the two denominators r1^3 and r2^3: each is the
-// correctly rounded quotient (hg_div_rn), i.e. the same bits as `/`.
+// The distances and the six quotients over r1^3 and r2^3 are formed on the
+// FP32 and integer pipes (hg_exact.cuh): the bits of sqrt and `/`, with 31
+// FP64 instructions left of 75.
 __device__ __forceinline__ void rhs6(const double (&s)[6], double mu, double (&d)[6]) {
   const double x = s[0], y = s[1], z = s[2], vx = s[3], vy = s[4];
   const double omu = 1.0 - mu;
   const double t1 = x + mu;
   const double yy = y * y;
   const double zz = z * z;
-  const double r1 = sqrt((t1 * t1 + yy) + zz);
+  const double r1 = hg_sqrt((t1 * t1 + yy) + zz);
   const double t2 = x - omu;
-  const double r2 = sqrt((t2 * t2 + yy) + zz);
+  const double r2 = hg_sqrt((t2 * t2 + yy) + zz);
   const double r1c = r1 * (r1 * r1);
   const double r2c = r2 * (r2 * r2);
-  const double i1 = hg_rcp_rn(r1c);
-  const double i2 = hg_rcp_rn(r2c);
+  const double n1[3] = {omu * t1, omu * y, (-omu) * z};
+  const double n2[3] = {mu * ((x - 1.0) + mu), mu * y, mu * z};
+  double q1[3], q2[3];
+  hg_quotients(n1, r1c, q1);
+  hg_quotients(n2, r2c, q2);
   d[0] = vx;
   d[1] = vy;
   d[2] = s[5];
-  d[3] = ((2.0 * vy + x) - hg_div_rn(omu * t1, r1c, i1)) - hg_div_rn(mu * ((x - 1.0) + mu), r2c, i2);
-  d[4] = ((-2.0 * vx + y) - hg_div_rn(omu * y, r1c, i1)) - hg_div_rn(mu * y, r2c, i2);
-  d[5] = hg_div_rn((-omu) * z, r1c, i1) - hg_div_rn(mu * z, r2c, i2);
+  d[3] = ((2.0 * vy + x) - q1[0]) - q2[0];
+  d[4] = ((-2.0 * vx + y) - q1[1]) - q2[1];
+  d[5] = q1[2] - q2[2];
 }
 
 // Hessian of the effective potential and the state accelerations,
@@ -218,12 +223,11 @@ __device__ __forceinline__ Hess hessian_split(const LT& L, int job, double x, do
   const double zs = L.from(sq, 4);
   const double rr = ((b2 ? t2s : t1s) + ys) + zs;
   const double den = hg_pow15_or_25(rr, k == 2);  // r^3 (jobs 0, 1) or r^5 (job 2) of the lane's primary
-  const double inv = hg_rcp_rn(den);
   const double mt = sq;  // jobs 2 and 5
-  const double n0 = k == 1 ? y : m;
-  const double n1 = k == 0 ? tt : (k == 1 ? z : mt);
-  const double q0 = hg_div_rn(n0, den, inv);
-  const double q1 = hg_div_rn(n1, den, inv);
+  const double num[2] = {k == 1 ? y : m, k == 0 ? tt : (k == 1 ? z : mt)};
+  double quo[2];
+  hg_quotients(num, den, quo);
+  const double q0 = quo[0], q1 = quo[1];
   // exchange: qa, qb, the r^3 terms of c3, the r^5 terms of sxy
   const double qa = L.from(q0, 2), qb = L.from(q0, 5);
   const double c3a = L.from(q0, 0), c3b = L.from(q0, 3);
@@ -420,12 +424,12 @@ struct Layout<2> {
     const double sqo = __shfl_xor_sync(gmask, sq, 1);
     const double yy = r0 ? sq : sqo;
     const double zz = r0 ? sqo : sq;
-    const double r = sqrt((t * t + yy) + zz);
+    const double r = hg_sqrt((t * t + yy) + zz);
     const double rc = r * (r * r);
-    const double ir = hg_rcp_rn(rc);
-    const double qx = hg_div_rn(mb * ((x + a1) + a2), rc, ir);
-    const double qy = hg_div_rn(mb * y, rc, ir);
-    const double qz = hg_div_rn(mz * z, rc, ir);
+    const double n[3] = {mb * ((x + a1) + a2), mb * y, mz * z};
+    double q[3];
+    hg_quotients(n, rc, q);
+    const double qx = q[0], qy = q[1], qz = q[2];
     // The accelerations ((2 vy + x) - q1x) - q2x and ((-2 vx + y) - q1y) - q2y
     // (q1 the first primary's quotient, role 0's; q2 the second's, role 1's)
     // in one instruction stream: role 0 forms ax, role 1 ay, and role 1
@@ -490,13 +494,15 @@ struct Layout<6> {
     const double tt = __shfl_sync(gmask, sq, base + (b0 ? 0 : 3));
     const double yy = __shfl_sync(gmask, sq, base + 1);
     const double zz = __shfl_sync(gmask, sq, base + 2);
-    const double r = sqrt((tt + yy) + zz);
+    const double r = hg_sqrt((tt + yy) + zz);
     const double rc = r * (r * r);
-    const double ir = hg_rcp_rn(rc);
     const double nx = (x + a1) + a2;
     const double nb = ax == 0 ? nx : (ax == 1 ? y : z);
     const double m = b0 ? (ax == 2 ? -omu : omu) : mu;
-    const double q = hg_div_rn(m * nb, rc, ir);
+    const double n[1] = {m * nb};
+    double qq[1];
+    hg_quotients(n, rc, qq);
+    const double q = qq[0];
     // first primary's quotient of this lane's axis (lanes 3..5 use it)
     const double pq = __shfl_sync(gmask, q, base + ax);
     const double c2 = role == 3 ? 2.0 : -2.0;
@@ -1870,16 +1876,18 @@ __global__ void __launch_bounds__(128) dop853_kernel(DopParams p) {
 #pragma unroll
         for (int d = 0; d < NC; ++d) {
           const double scale = p.atol + p.rtol * np_maximum_abs(y[d], yh[d]);
-          const double is = hg_rcp_rn(scale);
-          s5[d] = hg_div_rn(e5[d], scale, is);
-          s3[d] = hg_div_rn(e3[d], scale, is);
+          const double n53[2] = {e5[d], e3[d]};
+          double q53[2];
+          hg_quotients(n53, scale, q53);
+          s5[d] = q53[0];
+          s3[d] = q53[1];
         }
         double n5, n3;
         gat.dot2(L, s5, s3, n5, n3);
         if (hg_both0(n5, n3))
           err_norm = 0.0;
         else
-          err_norm = (fabs(h) * n5) / sqrt((n5 + 0.01 * n3) * (double)D);
+          err_norm = hg_div(fabs(h) * n5, hg_sqrt((n5 + 0.01 * n3) * (double)D));
       }
       const bool accepted = hg_le_pos(err_norm, HG_BITS_1);  // err_norm <= 1
       bool fin = true;

@@ -560,9 +560,11 @@ __device__ __forceinline__ bool pair_dop_run(const LT& L, const DopParams& p, Pa
 #pragma unroll
     for (int d = 0; d < NC; ++d) {
       const double scale = p.atol + p.rtol * np_maximum_abs(y[d], yh[d]);
-      const double is = hg_rcp_rn(scale);
-      s5[d] = hg_div_rn(e5[d], scale, is);
-      s3[d] = hg_div_rn(e3[d], scale, is);
+      const double n53[2] = {e5[d], e3[d]};
+      double q53[2];
+      hg_quotients(n53, scale, q53);
+      s5[d] = q53[0];
+      s3[d] = q53[1];
       fin = fin && finite_bits(yh[d]);
     }
     fin = __all_sync(L.gmask, fin);
@@ -573,7 +575,7 @@ __device__ __forceinline__ bool pair_dop_run(const LT& L, const DopParams& p, Pa
     if (hg_both0(n5, n3))
       err_norm = 0.0;
     else
-      err_norm = (fabs(hh) * n5) / sqrt((n5 + 0.01 * n3) * (double)D);
+      err_norm = hg_div(fabs(hh) * n5, hg_sqrt((n5 + 0.01 * n3) * (double)D));
     const bool accepted = hg_le_pos(err_norm, HG_BITS_1);  // err_norm <= 1
     const double t_new = t + hh;
     // dense samples inside (t, t_new] (reference: searchsorted on nodes);
