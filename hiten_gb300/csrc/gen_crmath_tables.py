@@ -5,7 +5,13 @@
 * log table: for F_j = 1 + j/1024, j in [LOG_JMIN, LOG_JMAX]:
   RN(1/F_j) and log(F_j) as a double-double (hi, lo);
 * exp table: 2^(j/256), j in [0, 256), as a double-double (hi, lo);
-* ln 2 split for the exponent term and ln2/256 split for argument reduction.
+* ln 2 split for the exponent term and ln2/256 split for argument reduction;
+
+and those of its integer form (``hg_powint.cuh``), in ``hg_powint_tables.h``:
+
+* r_j = ceil(2^16 / (1 + j/1024)) and round(-log2(r_j / 2^16) 2^64), j in [0, 1024);
+* round(2^(j/1024) 2^63), j in [0, 1024);
+* the coefficients of both polynomials in fixed point.
 
 Usage: ``python hiten_gb300/csrc/gen_crmath_tables.py`` (needs mpmath).
 """
@@ -77,5 +83,33 @@ def main():
         f.write("".join(out))
 
 
+def powint():
+    r, lg, ex = [], [], []
+    for j in range(1024):
+        r.append(-(-2**16 * 1024 // (1024 + j)))
+        lg.append(int(mp.nint(-mp.log(mp.mpf(r[-1]) / 2**16, 2) * mp.mpf(2)**64)))
+        ex.append(int(mp.nint(mp.power(2, mp.mpf(j) / 1024) * mp.mpf(2)**63)))
+
+    def arr(name, vals, fmt):
+        return f"#define {name}_INIT {{ \\\n  " + ", \\\n  ".join(
+            ", ".join(fmt % v for v in vals[i:i + 4]) for i in range(0, len(vals), 4)) + " }\n\n"
+
+    def fix(name, v, bits, suffix):
+        return f"#define {name} {hex(int(mp.nint(v * mp.mpf(2)**bits)))}{suffix}\n"
+
+    a = [None] + [1 / (k * mp.log(2)) for k in range(1, 7)]  # log2(1 + z) = z (a1 - z (a2 - z (a3 - ...)))
+    b = [None] + [mp.log(2)**k / mp.factorial(k) for k in range(1, 6)]  # 2^t - 1 = t (b1 + t (b2 + ...))
+    out = ["/* Generated by hiten_gb300/csrc/gen_crmath_tables.py (mpmath, 200 bits). */\n",
+           "#ifndef HG_POWINT_TABLES_H\n#define HG_POWINT_TABLES_H\n\n",
+           arr("HG_PI_R", r, "%d"), arr("HG_PI_L", lg, "0x%016xull"), arr("HG_PI_E", ex, "0x%016xull"),
+           fix("HG_PI_A1", a[1] / 2, 64, "ull"), fix("HG_PI_A2", a[2], 64, "ull"), fix("HG_PI_A3", a[3], 33, "u"),
+           fix("HG_PI_A4", a[4], 24, "u"), fix("HG_PI_A5", a[5] - a[6] / 2048, 15, "u"),
+           fix("HG_PI_B1", b[1], 64, "ull"), fix("HG_PI_B2", b[2], 66, "ull"), fix("HG_PI_B3", b[3], 36, "u"),
+           fix("HG_PI_B4", b[4], 26, "u"), fix("HG_PI_B5", b[5], 16, "u"), "\n#endif\n"]
+    with open(os.path.join(HERE, "hg_powint_tables.h"), "w") as f:
+        f.write("".join(out))
+
+
 if __name__ == "__main__":
     main()
+    powint()

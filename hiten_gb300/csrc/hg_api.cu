@@ -126,12 +126,20 @@ int lanes_d42_dop_free(const hg_handle* h, int n) {
   return 3.0 * ((n + hg::kPairTraj - 1) / hg::kPairTraj) <= cap ? 18 : 12;
 }
 
+// Allow a kernel more dynamic shared memory than a launch gets unasked.
+template <class K>
+bool allow_smem(K kernel, size_t bytes) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
+}
+
 // Paired-warp DOP853 launch (42-dim, no event, single pass): blocks of one
 // pair (two with HG_TUNE_BLOCK_THREADS 128).
 int launch_dop853_trio(hg_handle* h, const hg::DopParams& p, cudaStream_t s) {
   const int grid = (p.N + hg::kPairTraj - 1) / hg::kPairTraj;
   if (grid < 1) return HG_OK;
-  hg::dop853_trio_kernel<<<grid, 96, 0, s>>>(p);
+  hg::dop853_trio_kernel<<<grid, 96, hg::trio_dop_smem(), s>>>(p);
   return check_launch(h, "dop853_trio_kernel");
 }
 
@@ -140,7 +148,9 @@ int launch_dop853_pair(hg_handle* h, const hg::DopParams& p, cudaStream_t s) {
   const int per_block = (block / 64) * hg::kPairTraj;
   const int grid = (p.N + per_block - 1) / per_block;
   if (grid < 1) return HG_OK;
-  hg::dop853_pair_kernel<<<grid, block, 0, s>>>(p);
+  const size_t smem = hg::pair_dop_smem(block);
+  if (block > 64 && !allow_smem(hg::dop853_pair_kernel, smem)) return fail(h, HG_ERR_CUDA, "shared memory");
+  hg::dop853_pair_kernel<<<grid, block, smem, s>>>(p);
   return check_launch(h, "dop853_pair_kernel");
 }
 
@@ -154,15 +164,10 @@ int launch_fixed_pair(hg_handle* h, const hg::FixedParams& p, cudaStream_t s) {
   const int per_block = (block / 64) * hg::kPairTraj;
   const int grid = (p.N + per_block - 1) / per_block;
   if (grid < 1) return HG_OK;
-  size_t smem = 0;
-  if (block == 128 && grid <= h->sm_count && h->smem_per_sm > 0) {
-    smem = (size_t)(h->smem_per_sm / 2 + 1024);
-    if (cudaFuncSetAttribute(hg::fixed_rk_pair_kernel<ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess) {
-      cudaGetLastError();
-      smem = 0;
-    }
-  }
+  size_t smem = hg::pair_fixed_smem<ORDER>(block);
+  const size_t half = (size_t)(h->smem_per_sm / 2 + 1024);
+  if (block == 128 && grid <= h->sm_count && half > smem) smem = half;
+  if (block > 64 && !allow_smem(hg::fixed_rk_pair_kernel<ORDER>, smem)) return fail(h, HG_ERR_CUDA, "shared memory");
   hg::fixed_rk_pair_kernel<ORDER><<<grid, block, smem, s>>>(p);
   return check_launch(h, "fixed_rk_pair_kernel");
 }
@@ -172,7 +177,7 @@ template <int ORDER>
 int launch_fixed_trio(hg_handle* h, const hg::FixedParams& p, cudaStream_t s) {
   const int grid = (p.N + hg::kPairTraj - 1) / hg::kPairTraj;
   if (grid < 1) return HG_OK;
-  hg::fixed_rk_trio_kernel<ORDER><<<grid, 96, 0, s>>>(p);
+  hg::fixed_rk_trio_kernel<ORDER><<<grid, 96, hg::trio_fixed_smem<ORDER>(), s>>>(p);
   return check_launch(h, "fixed_rk_trio_kernel");
 }
 
@@ -308,17 +313,19 @@ struct Shape {
   int per_sm;
 };
 
-template <class K>
+template <int G, class K>
 Shape dop_shape(const hg_handle* h, K kernel) {
-  Shape sh{h->block, 0, 1};
+  Shape sh{h->block, hg::dop_smem_bytes<G>(h->block), 1};
   if (h->spread && h->smem_per_sm > 0) {
+    const size_t half = (size_t)(h->smem_per_sm / 2 + 1024);
     sh.block = 128;
-    sh.smem = (size_t)(h->smem_per_sm / 2 + 1024);
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem) != cudaSuccess) {
-      cudaGetLastError();
-      sh.block = h->block;
-      sh.smem = 0;
-    }
+    sh.smem = hg::dop_smem_bytes<G>(128) > half ? hg::dop_smem_bytes<G>(128) : half;
+  }
+  if (sh.smem > 32 * 1024 &&  // with the static part above the 48 KB a launch gets unasked
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem) != cudaSuccess) {
+    cudaGetLastError();
+    sh.block = 32;  // fits without the attribute
+    sh.smem = hg::dop_smem_bytes<G>(32);
   }
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, sh.block, sh.smem) != cudaSuccess ||
@@ -335,7 +342,7 @@ int launch_dop853(hg_handle* h, hg::DopParams p, cudaStream_t s) {
   if (p.N <= 0) return HG_OK;
   // launches without dense samples run the kernel built without that path
   auto kern = p.m >= 2 ? hg::dop853_kernel<G, true> : hg::dop853_kernel<G, false>;
-  const Shape sh = dop_shape(h, kern);
+  const Shape sh = dop_shape<G>(h, kern);
   const int kBlock = sh.block;
   const int per_sm = sh.per_sm;
   cudaError_t e;
@@ -415,7 +422,7 @@ long long seg_ws_layout(int N, int D, int max_hits, char* base, SegWs* w) {
 template <int G>
 int launch_segment(hg_handle* h, hg::DopParams p, const SegWs& w, int seg_steps, int a, int n_live, cudaStream_t s) {
   auto kern = p.m >= 2 ? hg::dop853_kernel<G, true> : hg::dop853_kernel<G, false>;
-  const Shape sh = dop_shape(h, kern);
+  const Shape sh = dop_shape<G>(h, kern);
   const int kBlock = sh.block;
   const int per_sm = sh.per_sm;
   const int tpb = (kBlock / 32) * hg::Layout<G>::TPW;

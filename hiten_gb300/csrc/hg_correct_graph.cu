@@ -565,9 +565,9 @@ struct Dev {
 };
 
 template <class K>
-int resident_blocks(K kern, int block, int sms) {
+int resident_blocks(K kern, int block, int sms, size_t smem = 0) {
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, 0) != cudaSuccess || per_sm < 1) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     per_sm = 1;
   }
@@ -628,10 +628,10 @@ void event_leg(const Ws& w, double mu, const hg_newton_opts& o, int sms, cudaStr
   p.rec_ld = capr;
   const int tpb = hg::Layout<G>::TPW;
   const int need = (w.cap + tpb - 1) / tpb;
-  const int cap_blocks = resident_blocks(hg::dop853_kernel<G, false>, 32, sms);
+  const int cap_blocks = resident_blocks(hg::dop853_kernel<G, false>, 32, sms, hg::dop_smem_bytes<G>(32));
   const int grid = need < cap_blocks ? need : cap_blocks;
   p.stride = grid * tpb;
-  hg::dop853_kernel<G, false><<<grid, 32, 0, s>>>(p);
+  hg::dop853_kernel<G, false><<<grid, 32, hg::dop_smem_bytes<G>(32), s>>>(p);
   // refinement of the saved crossings (records [0, refine_count))
   const int rneed = (int)((capr + 31) / 32);
   const int rcap = resident_blocks(hg::refine_kernel<1>, 32, sms);
@@ -686,16 +686,16 @@ void stm_leg(const Ws& w, double mu, const hg_newton_opts& o, int sms, cudaStrea
     // block, the live count read from n_in (their list is the identity)
     const int grid = (w.cap + hg::kPairTraj - 1) / hg::kPairTraj;
     if constexpr (G == 18)
-      hg::dop853_trio_kernel<<<grid, 96, 0, s>>>(p);
+      hg::dop853_trio_kernel<<<grid, 96, hg::trio_dop_smem(), s>>>(p);
     else
-      hg::dop853_pair_kernel<<<grid, 64, 0, s>>>(p);
+      hg::dop853_pair_kernel<<<grid, 64, hg::pair_dop_smem(64), s>>>(p);
   } else {
     const int tpb = hg::Layout<G>::TPW;
     const int need = (w.cap + tpb - 1) / tpb;
-    const int cap_blocks = resident_blocks(hg::dop853_kernel<G, true>, 32, sms);
+    const int cap_blocks = resident_blocks(hg::dop853_kernel<G, true>, 32, sms, hg::dop_smem_bytes<G>(32));
     const int grid = need < cap_blocks ? need : cap_blocks;
     p.stride = grid * tpb;
-    hg::dop853_kernel<G, true><<<grid, 32, 0, s>>>(p);
+    hg::dop853_kernel<G, true><<<grid, 32, hg::dop_smem_bytes<G>(32), s>>>(p);
   }
   *launches += 1;
 }

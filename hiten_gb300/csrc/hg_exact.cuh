@@ -224,7 +224,8 @@ HG_XHD float hgx_sqrt_arg(double x) {
 //     with an error of at most 990 * 2^-22.9 (y) + 2.1e-4 (FP32 sums) <
 //     3.4e-4, so where it is more than 4e-4 from a half, c2 rounded is the
 //     nearest.
-HG_XHD double hgx_sqrt(double x, float y, bool& ok) {
+// S_raw: S + 2^32 HGX_OFFSET; fr: sqrt(a 2^52) - S, off by at most 3.4e-4.
+HG_XHD void hgx_sqrt_parts(double x, float y, uint64_t& S_raw, float& fr) {
   const uint32_t hi = hgx_hi(x), lo = hgx_lo(x);
   const uint32_t sh = (hi >> 20) & 1u;  // 1: a is the significand, 0: twice it
   const uint32_t alo = lo << (1u - sh);
@@ -241,8 +242,14 @@ HG_XHD double hgx_sqrt(double x, float y, bool& ok) {
   const float f2 = fmaf(c1f, c1f * -0x1p-14f, (float)ri);
   const float yk = y * 0x1p-19f;
   const float v = fmaf(f2, yk, HGX_M2);
-  const float fr = fmaf(f2, yk, -(v - HGX_M2));
-  const uint64_t S = hgx_mad_wide_u(sb, 1u << 29, hgx_mad_wide_u(b1, 1024u, hgx_fbits(v)));
+  fr = fmaf(f2, yk, -(v - HGX_M2));
+  S_raw = hgx_mad_wide_u(sb, 1u << 29, hgx_mad_wide_u(b1, 1024u, hgx_fbits(v)));
+}
+HG_XHD double hgx_sqrt(double x, float y, bool& ok) {
+  uint64_t S;
+  float fr;
+  hgx_sqrt_parts(x, y, S, fr);
+  const uint32_t hi = hgx_hi(x);
   ok = hgx_positive_in_range(hi) && fabsf(fr) < 0.4996f;
   const uint32_t ex = ((hi + (1021u << 20)) >> 1) & 0x7FF00000u;
   return hgx_make((uint32_t)(S >> 32) + (ex - HGX_OFFSET), (uint32_t)S);

@@ -33,6 +33,7 @@
 
 #include "hg_crmath.cuh"
 #include "hg_exact.cuh"
+#include "hg_powint.cuh"
 #include "hg_tableaux.h"
 #include "hitengpu.h"
 
@@ -192,8 +193,8 @@ struct Layout<1> {
 // hessian42 with its work spread over a lane group: lane base + job does job
 // (0..5); L.from(v, r) reads lane base + r.  Lane b*3 + k (b = primary,
 // k < 3) takes the power of its primary its quotients divide by (r^3 for
-// k < 2, r^5 for k = 2; hg_pow15_or_25), one reciprocal and two of the
-// twelve quotients:
+// k < 2, r^5 for k = 2) and two of the twelve quotients, on the FP32 and
+// integer pipes (hg_powint.cuh, hg_exact.cuh):
 //   0: mu2/r3, t1/r3     1: y/r3, z/r3     2: mu2/r5, (mu2 t1)/r5
 //   3: mu/R3,  t2/R3     4: y/R3, z/R3     5: mu/R5,  (mu t2)/R5
 // (further lanes repeat job 0).  The quotients are exchanged, lanes 0..5
@@ -749,26 +750,40 @@ __device__ __forceinline__ double exp_scaled(double e, double Lh, double Ll) {
 // [0.2, 10].  Accepting and rejecting lanes share the logarithm, so a warp
 // whose trajectories disagree runs one transcendental sequence, not two; in
 // a group of lanes the two exponentials run on two lanes at once.  Every
-// power is the correctly rounded one hg_pow gives.  Zero, NaN and
+// power is the correctly rounded one, formed on the integer pipes
+// (hg_powint.cuh; the double-double form decides the rest).  Zero, NaN and
 // err >= 1e300 take no logarithm: their factors are the clamp bounds (a
 // rejected err >= 1e300 gives 0.9 * err^(-1/8) < 0.2).
 template <class LT>
 __device__ __forceinline__ double pi_factor(const LT& L, bool accepted, double err, double err_prev,
                                             double& prev_pow) {
-  const double beta = 1.0 / (8.0 + 1.0);
-  const double alpha = 0.4 * beta;
-  const double rexp = 1.0 / 8.0;
+  constexpr double beta = 1.0 / (8.0 + 1.0);
+  constexpr double alpha = 0.4 * beta;
+  constexpr double rexp = 1.0 / 8.0;
   const bool regular = hg_in_open_pos(err, HG_BITS_1E300);  // 0 < err < 1e300
   double p1 = 0.0, pa = 0.0;
   if (regular) {
-    double Lh, Ll;
-    hg_log_dd(err, Lh, Ll);
+    const HgLog2 lg = hgp_log2(err);
     const double e1 = accepted ? -beta : -rexp;
+    constexpr uint64_t Yb = (uint64_t)(beta * 0x1p64), Yr = (uint64_t)(rexp * 0x1p64), Ya = (uint64_t)(alpha * 0x1p64);
     if constexpr (std::is_same_v<LT, Layout<1>>) {
-      p1 = exp_scaled(e1, Lh, Ll);
-      pa = exp_scaled(alpha, Lh, Ll);
+      bool o1, oa;
+      p1 = hgp_exp(lg, accepted ? Yb : Yr, true, o1);
+      pa = hgp_exp(lg, Ya, false, oa);
+      if (!(o1 && oa)) {
+        double Lh, Ll;
+        hg_log_dd(err, Lh, Ll);
+        p1 = exp_scaled(e1, Lh, Ll);
+        pa = exp_scaled(alpha, Lh, Ll);
+      }
     } else {
-      const double v = exp_scaled(L.role == 0 ? e1 : alpha, Lh, Ll);
+      bool ok;
+      double v = hgp_exp(lg, L.role == 0 ? (accepted ? Yb : Yr) : Ya, L.role == 0, ok);
+      if (!ok) {
+        double Lh, Ll;
+        hg_log_dd(err, Lh, Ll);
+        v = exp_scaled(L.role == 0 ? e1 : alpha, Lh, Ll);
+      }
       p1 = __shfl_sync(L.gmask, v, L.base);
       pa = __shfl_sync(L.gmask, v, L.base + 1);
     }
@@ -818,6 +833,116 @@ __device__ __forceinline__ double np_maximum_abs(double a, double b) {
 // isfinite on the integer pipe (exponent field not all ones).
 __device__ __forceinline__ bool finite_bits(double a) {
   return ((unsigned long long)__double_as_longlong(a) & 0x7FF0000000000000ull) != 0x7FF0000000000000ull;
+}
+
+// ---------------------------------------------------------------------------
+// The steps as loops over the stages
+// ---------------------------------------------------------------------------
+// With its integer sequences a right-hand side is several hundred
+// instructions; one unrolled copy per stage makes a step larger than the
+// instruction cache, and a warp alone then runs at the rate of the fetches.
+// So the stages are a loop over the tableau's nonzero entries, listed by
+// rows: entry q is coefficient c[q] of derivative col[q]; row i (0 .. S - 1
+// the stages, S the weights) is [row[i], row[i + 1]).  Each sum has the terms
+// and the order of the unrolled form, so the bits too.
+template <int S>
+struct StageList {
+  static constexpr int kMax = (S + 1) * (S + 2) / 2;
+  double c[kMax];
+  int col[kMax];
+  int row[S + 2];
+};
+template <class T>
+__host__ __device__ constexpr StageList<T::S> make_stage_list() {
+  StageList<T::S> t{};
+  int q = 0;
+  for (int i = 0; i <= T::S; ++i) {
+    t.row[i] = q;
+    for (int j = 0; j < i; ++j) {
+      const double v = i < T::S ? T::a(i, j) : T::b(j);
+      if (v != 0.0) {
+        t.c[q] = v;
+        t.col[q++] = j;
+      }
+    }
+  }
+  t.row[T::S + 1] = q;
+  return t;
+}
+template <class T>
+__host__ __device__ constexpr int stage_nnz() {
+  return make_stage_list<T>().row[T::S + 1];
+}
+__device__ __constant__ static const StageList<4> hg_list_rk4 = make_stage_list<FixedTab<4>>();
+__device__ __constant__ static const StageList<7> hg_list_rk6 = make_stage_list<FixedTab<6>>();
+__device__ __constant__ static const StageList<13> hg_list_rk8 = make_stage_list<FixedTab<8>>();
+__device__ __constant__ static const StageList<12> hg_list_dop = make_stage_list<DopTab>();
+template <class T>
+__device__ __forceinline__ const StageList<T::S>& stage_list() {
+  if constexpr (std::is_same_v<T, DopTab>)
+    return hg_list_dop;
+  else if constexpr (std::is_same_v<T, FixedTab<8>>)
+    return hg_list_rk8;
+  else if constexpr (std::is_same_v<T, FixedTab<6>>)
+    return hg_list_rk6;
+  else
+    return hg_list_rk4;
+}
+
+// The stage derivatives of a lane's components in shared memory,
+// lane-contiguous: derivative j, component d of a warp are 32 doubles.
+template <int NC>
+struct StageRow {
+  double* q;
+  __device__ __forceinline__ double& operator[](int d) const { return q[d * 32]; }
+};
+template <int NC>
+struct StageMem {
+  double* p;
+  __device__ __forceinline__ StageRow<NC> operator[](int j) const { return StageRow<NC>{p + j * (NC * 32)}; }
+};
+
+// The products h c[q].  ListCoef: formed where they are used (one lane per
+// trajectory).  TableCoef: formed once per step into shared memory by the
+// lanes that share the step size (a group of NL lanes or a whole warp), entry
+// q at tab[q * STRIDE]; lanes of several groups interleave their entries.
+template <class T>
+struct ListCoef {
+  double h;
+  __device__ __forceinline__ void set_step(double hh) { h = hh; }
+  __device__ __forceinline__ double product(int q) const { return h * stage_list<T>().c[q]; }
+};
+template <class T, int NL, int STRIDE>
+struct TableCoef {
+  double* tab;
+  int r;
+  unsigned gmask;
+  __device__ __forceinline__ void set_step(double h) {
+    __syncwarp(gmask);  // the group has read the last step's
+#pragma unroll 1
+    for (int q = r; q < stage_nnz<T>(); q += NL) tab[q * STRIDE] = h * stage_list<T>().c[q];
+    __syncwarp(gmask);
+  }
+  __device__ __forceinline__ double product(int q) const { return tab[q * STRIDE]; }
+};
+
+// y + sum of row i's products: the argument of stage i, or (i = S) the step's
+// end.  (Loading the next entry's operands under this one's sum was measured
+// too: 3 % slower for one and two lanes, level for six.)
+template <class T, int NC, class CF>
+__device__ __forceinline__ void stage_sum(int i, const double (&y)[NC], const CF& cf, const StageMem<NC>& k,
+                                          double (&ys)[NC]) {
+  const StageList<T::S>& tl = stage_list<T>();
+#pragma unroll
+  for (int d = 0; d < NC; ++d) ys[d] = y[d];
+  const int end = tl.row[i + 1];
+#pragma unroll 1
+  for (int q = tl.row[i]; q < end; ++q) {
+    const StageRow<NC> kr = k[tl.col[q]];
+    const double c = cf.product(q);
+#pragma unroll
+    for (int d = 0; d < NC; ++d) ys[d] = ys[d] + c * kr[d];
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -943,6 +1068,24 @@ __device__ __forceinline__ void rk_fixed_step(const LT& L, const double (&y)[LT:
       for (int d = 0; d < NC; ++d) yn[d] = yn[d] + c * k[j][d];
     }
   });
+}
+
+// The same step with the stages as a loop.
+template <int ORDER, class LT, class CF>
+__device__ __forceinline__ void rk_fixed_step_loop(const LT& L, const double (&y)[LT::NC], const CF& cf, double mu,
+                                                   const Dir& dir, const StageMem<LT::NC>& k, double (&yn)[LT::NC]) {
+  using T = FixedTab<ORDER>;
+  constexpr int NC = LT::NC;
+#pragma unroll 1
+  for (int i = 0; i < T::S; ++i) {
+    double ys[NC], kt[NC];
+    stage_sum<T>(i, y, cf, k, ys);
+    L.rhs(ys, mu, dir, kt);
+    const StageRow<NC> kr = k[i];
+#pragma unroll
+    for (int d = 0; d < NC; ++d) kr[d] = kt[d];
+  }
+  stage_sum<T>(T::S, y, cf, k, yn);
 }
 
 template <int ORDER, class LT>
@@ -1319,115 +1462,20 @@ struct DopGroupCoef {
   }
 };
 
-// Row I of the step's coefficients (I < 12: the stage row a_Ij; I = 12: the
-// solution weights b_j), its count of nonzero entries and the column of the
-// k-th of them.
-template <int I>
-__host__ __device__ constexpr double dop_row_coef(int j) {
-  return I < DopTab::S ? DopTab::a(I, j) : DopTab::b(j);
-}
-template <int I>
-__host__ __device__ constexpr int dop_row_nnz() {
-  int n = 0;
-  for (int j = 0; j < (I < DopTab::S ? I : DopTab::S); ++j) n += dop_row_coef<I>(j) != 0.0;
-  return n;
-}
-template <int I>
-__host__ __device__ constexpr int dop_row_col(int k) {
-  for (int j = 0; j < (I < DopTab::S ? I : DopTab::S); ++j)
-    if (dop_row_coef<I>(j) != 0.0 && k-- == 0) return j;
-  return -1;
-}
-
-// Lane pairs (G = 2, one step size per pair): the products h * a_ij, h * b_j
-// formed row by row at the start of each stage, two per FP64 multiply --
-// lane `role` of the pair forms the (2m + role)-th nonzero entry of the row
-// -- and exchanged by shuffle: the same products as DopInlineCoef in about
-// half the multiplies.  `c` holds the current row's products by column.
-struct DopPairCoef {
-  double h;
-  int role;
-  int base;
-  unsigned gmask;
-  mutable double c[DopTab::S];
-  __device__ __forceinline__ void set_step(double hh) { h = hh; }
-  template <int I>
-  __device__ __forceinline__ void row() const {
-    constexpr int n = dop_row_nnz<I>();
-    static_for<(n + 1) / 2>([&](auto mc) {
-      constexpr int m = decltype(mc)::value;
-      constexpr int ja = dop_row_col<I>(2 * m);
-      constexpr int jb = 2 * m + 1 < n ? dop_row_col<I>(2 * m + 1) : -1;
-      constexpr double aa = dop_row_coef<I>(ja);
-      constexpr double ab = jb >= 0 ? dop_row_coef<I>(jb) : aa;
-      const double v = h * (role ? ab : aa);
-      c[ja] = __shfl_sync(gmask, v, base);
-      if constexpr (jb >= 0) c[jb] = __shfl_sync(gmask, v, base + 1);
-    });
-  }
-  template <int I, int J>
-  __device__ __forceinline__ double a() const {
-    return c[J];
-  }
-  template <int J>
-  __device__ __forceinline__ double b() const {
-    return c[J];
-  }
+template <int NC>
+struct StageRegs {
+  double v[13][NC];
+  __device__ __forceinline__ double (&operator[](int j))[NC] { return v[j]; }
+  __device__ __forceinline__ const double (&operator[](int j) const)[NC] { return v[j]; }
 };
-
-// Row preparation of a coefficient provider: DopPairCoef forms a row's
-// products ahead of its sum; the others form them where they are used.
-template <int I, class CF>
-__device__ __forceinline__ void dop_coef_row(const CF&) {}
-template <int I>
-__device__ __forceinline__ void dop_coef_row(const DopPairCoef& cf) {
-  cf.template row<I>();
-}
 
 template <class LT>
 struct DopLaneT {
   static constexpr int NC = LT::NC;
-  // one attempted DOP853 step; k[0] = f(t, y) on entry; k[12] = f(t+h, y_high)
-  // on exit.
-  __device__ __forceinline__ static void step(const LT& L, const double (&y)[NC], double h, double mu,
-                                              const Dir& dir, double (&k)[13][NC], double (&yh)[NC],
-                                              double (&e5)[NC], double (&e3)[NC]) {
-    step(L, y, DopInlineCoef{h}, h, mu, dir, k, yh, e5, e3);
-  }
-  // the same with the products h * a_ij, h * b_j from `cf` (set for h)
-  template <class CF>
-  __device__ __forceinline__ static void step(const LT& L, const double (&y)[NC], const CF& cf, double h, double mu,
-                                              const Dir& dir, double (&k)[13][NC], double (&yh)[NC],
-                                              double (&e5)[NC], double (&e3)[NC]) {
+  // err5 / err3 of a step, from k[0..12]
+  template <class K>
+  __device__ __forceinline__ static void error_sums(const K& k, double h, double (&e5)[NC], double (&e3)[NC]) {
     using T = DopTab;
-    static_for<T::S - 1>([&](auto ic) {
-      constexpr int i = decltype(ic)::value + 1;
-      dop_coef_row<i>(cf);
-      double ys[NC];
-#pragma unroll
-      for (int d = 0; d < NC; ++d) ys[d] = y[d];
-      static_for<i>([&](auto jc) {
-        constexpr int j = decltype(jc)::value;
-        if constexpr (T::a(i, j) != 0.0) {
-          const double c = cf.template a<i, j>();
-#pragma unroll
-          for (int d = 0; d < NC; ++d) ys[d] = ys[d] + c * k[j][d];
-        }
-      });
-      L.rhs(ys, mu, dir, k[i]);
-    });
-    dop_coef_row<T::S>(cf);
-#pragma unroll
-    for (int d = 0; d < NC; ++d) yh[d] = y[d];
-    static_for<T::S>([&](auto jc) {
-      constexpr int j = decltype(jc)::value;
-      if constexpr (T::b(j) != 0.0) {
-        const double c = cf.template b<j>();
-#pragma unroll
-        for (int d = 0; d < NC; ++d) yh[d] = yh[d] + c * k[j][d];
-      }
-    });
-    L.rhs(yh, mu, dir, k[12]);
     // err5 = sum_j E5_j k_j (the reference starts from zeros; the first term
     // is taken as the start here: only the sign of an all-zero sum can
     // differ, and err5 / err3 enter the step control squared)
@@ -1453,11 +1501,64 @@ struct DopLaneT {
     }
   }
 
+  // One attempted step with the stages as a loop: k[0] on entry, k[1..12] on
+  // exit.
+  template <class CF>
+  __device__ __forceinline__ static void step_loop(const LT& L, const double (&y)[NC], const CF& cf, double h,
+                                                   double mu, const Dir& dir, const StageMem<NC>& k,
+                                                   double (&yh)[NC], double (&e5)[NC], double (&e3)[NC]) {
+#pragma unroll 1
+    for (int i = 1; i <= DopTab::S; ++i) {
+      stage_sum<DopTab>(i, y, cf, k, yh);
+      double kt[NC];
+      L.rhs(yh, mu, dir, kt);
+      const StageRow<NC> kr = k[i];
+#pragma unroll
+      for (int d = 0; d < NC; ++d) kr[d] = kt[d];
+    }
+    error_sums(k, h, e5, e3);
+  }
+  // one attempted DOP853 step; k[0] = f(t, y) on entry; k[12] = f(t+h, y_high)
+  // on exit; the products h * a_ij, h * b_j from `cf` (set for h)
+  template <class CF>
+  __device__ __forceinline__ static void step(const LT& L, const double (&y)[NC], const CF& cf, double h, double mu,
+                                              const Dir& dir, double (&k)[13][NC], double (&yh)[NC],
+                                              double (&e5)[NC], double (&e3)[NC]) {
+    using T = DopTab;
+    static_for<T::S - 1>([&](auto ic) {
+      constexpr int i = decltype(ic)::value + 1;
+      double ys[NC];
+#pragma unroll
+      for (int d = 0; d < NC; ++d) ys[d] = y[d];
+      static_for<i>([&](auto jc) {
+        constexpr int j = decltype(jc)::value;
+        if constexpr (T::a(i, j) != 0.0) {
+          const double c = cf.template a<i, j>();
+#pragma unroll
+          for (int d = 0; d < NC; ++d) ys[d] = ys[d] + c * k[j][d];
+        }
+      });
+      L.rhs(ys, mu, dir, k[i]);
+    });
+#pragma unroll
+    for (int d = 0; d < NC; ++d) yh[d] = y[d];
+    static_for<T::S>([&](auto jc) {
+      constexpr int j = decltype(jc)::value;
+      if constexpr (T::b(j) != 0.0) {
+        const double c = cf.template b<j>();
+#pragma unroll
+        for (int d = 0; d < NC; ++d) yh[d] = yh[d] + c * k[j][d];
+      }
+    });
+    L.rhs(yh, mu, dir, k[12]);
+    error_sums(k, h, e5, e3);
+  }
+
   // _dop853_build_dense_cache: F[0..6][6] for this lane's components.
+  template <class K>
   __device__ __forceinline__ static void dense_cache(const LT& L, const double (&y_old)[NC],
                                                      const double (&y_new)[NC], double hseg, double mu,
-                                                     const Dir& dir, const double (&k)[13][NC],
-                                                     double (&F)[7][NC]) {
+                                                     const Dir& dir, const K& k, double (&F)[7][NC]) {
     using T = DopTab;
     double kx[3][NC];
     static_for<3>([&](auto sc) {
@@ -1537,27 +1638,37 @@ struct DopLaneT {
 template <int G>
 using DopLane = DopLaneT<Layout<G>>;
 
-// Step-coefficient provider of a layout: spread over the group for the
-// groups of 6 and 14 lanes (few components per lane), formed row by row in
-// pairs for lane pairs, formed inline for 1 and 7 (whose lanes have no
-// registers to spare).
+// Layouts whose step is the looped form (stage derivatives in shared memory):
+// the ones whose lanes hold several components.  A six-lane or 42-dim group's
+// step is bound by the latency of its chain, to which the loop's address and
+// shared-memory latencies add (six lanes: 12 % on 1237 manifold seeds).
 template <int G>
-__host__ __device__ constexpr bool dop_spread_coef() {
-  return G == 6 || G == 14;
+__host__ __device__ constexpr bool dop_looped() {
+  return G == 1 || G == 2;
+}
+
+// Dynamic shared memory of a dop853_kernel<G> warp in the looped form: stage
+// derivatives, then (G > 1) the step's products.
+template <int G>
+__host__ __device__ constexpr int dop_warp_doubles() {
+  return dop_looped<G>() ? 13 * Layout<G>::NC * 32 + (G > 1 ? dop_nnz() * Layout<G>::TPW : 0) : 0;
 }
 template <int G>
-__device__ __forceinline__ auto dop_coef(const Layout<G>& L, const double* tab) {
-  if constexpr (dop_spread_coef<G>()) {
-    return DopGroupCoef<G>(tab, L.role, L.base, L.gmask);
-  } else if constexpr (G == 2) {
-    DopPairCoef cf;
-    cf.h = 0.0;
-    cf.role = L.role;
-    cf.base = L.base;
-    cf.gmask = L.gmask;
-    return cf;
+__host__ __device__ constexpr size_t dop_smem_bytes(int block) {
+  return (size_t)(block / 32) * dop_warp_doubles<G>() * sizeof(double);
+}
+
+template <int G>
+__device__ __forceinline__ auto dop_coef(const Layout<G>& L, const double* tab, double* sm_step) {
+  if constexpr (G == 1) {
+    return ListCoef<DopTab>{0.0};
+  } else if constexpr (dop_looped<G>()) {
+    double* const t = sm_step + (threadIdx.x >> 5) * dop_warp_doubles<G>() + 13 * Layout<G>::NC * 32;
+    return TableCoef<DopTab, G, Layout<G>::TPW>{t + (threadIdx.x & 31) / G, L.role, L.gmask};
+  } else if constexpr (G == 7) {
+    return DopInlineCoef{0.0};  // no registers to spare for the shares
   } else {
-    return DopInlineCoef{0.0};
+    return DopGroupCoef<G>(tab, L.role, L.base, L.gmask);
   }
 }
 
@@ -1686,10 +1797,10 @@ __device__ __forceinline__ int leader_lane(const Layout<G>& L) {
     return L.base;
 }
 
-template <int G>
+template <int G, class K>
 __device__ __forceinline__ void save_step(const Layout<G>& L, const DopParams& p, int traj, int hit, bool leader,
                                           const double (&y)[Layout<G>::NC], const double (&yh)[Layout<G>::NC],
-                                          const double (&k)[13][Layout<G>::NC], double h, double t, double g_left) {
+                                          const K& k, double h, double t, double g_left) {
   constexpr int D = Layout<G>::D;
   constexpr int NC = Layout<G>::NC;
   int slot = 0;
@@ -1765,8 +1876,9 @@ __global__ void __launch_bounds__(128) dop853_kernel(DopParams p) {
   Gather<G> gat;
   int traj;
   __shared__ double sm_gather[gather_smem_doubles<G>()];  // 4 warps x 4 groups
-  __shared__ double sm_coef[dop_spread_coef<G>() ? dop_nnz() : 1];
-  if constexpr (dop_spread_coef<G>()) {
+  __shared__ double sm_coef[dop_looped<G>() ? 1 : dop_nnz()];
+  extern __shared__ double sm_step[];  // dop_smem_bytes<G>(blockDim.x)
+  if constexpr (!dop_looped<G>()) {
     dop_coef_table_init(sm_coef);
     __syncthreads();
   }
@@ -1774,7 +1886,9 @@ __global__ void __launch_bounds__(128) dop853_kernel(DopParams p) {
   const bool leader = is_leader<G>(L);
   const bool has_event = p.ev_index >= 0 && p.max_hits > 0;
   const EvCtx<G> ev(L, has_event ? p.ev_index : -1);
-  auto cf = dop_coef<G>(L, sm_coef);
+  std::conditional_t<dop_looped<G>(), StageMem<NC>, StageRegs<NC>> k;
+  auto cf = dop_coef<G>(L, sm_coef, sm_step);
+  if constexpr (dop_looped<G>()) k.p = sm_step + (threadIdx.x >> 5) * dop_warp_doubles<G>() + (threadIdx.x & 31);
 
   const int slot0 = traj;
   int slot = traj;
@@ -1808,9 +1922,11 @@ __global__ void __launch_bounds__(128) dop853_kernel(DopParams p) {
 #pragma unroll
       for (int r = 0; r < NC; ++r) y[r] = p.y0[(long long)L.comp(r) * p.ld + traj];
     }
-    double k[13][NC];
+    double k0[NC];
     // on resume this is bitwise k[12] of the last accepted step
-    L.rhs(y, p.mu, p.dir, k[0]);
+    L.rhs(y, p.mu, p.dir, k0);
+#pragma unroll
+    for (int d = 0; d < NC; ++d) k[0][d] = k0[d];
     double g_prev = 0.0;
     if (has_event) g_prev = ev.bcast(ev.mine ? (pick<NC>(y, ev.r) - p.ev_offset) : 0.0);
     double h, t, err_prev, prev_pow;
@@ -1831,7 +1947,7 @@ __global__ void __launch_bounds__(128) dop853_kernel(DopParams p) {
       for (int d = 0; d < NC; ++d) {
         const double scale0 = p.atol + p.rtol * fabs(y[d]);
         a[d] = y[d] / scale0;
-        b[d] = k[0][d] / scale0;
+        b[d] = k0[d] / scale0;
       }
       const double sn = sqrt((double)D);
       double na, nb;
@@ -1869,7 +1985,10 @@ __global__ void __launch_bounds__(128) dop853_kernel(DopParams p) {
       h = adjust_step_to_endpoint(t, h, tmax);
       double yh[NC], e5[NC], e3[NC];
       cf.set_step(h);
-      DopLane<G>::step(L, y, cf, h, p.mu, p.dir, k, yh, e5, e3);
+      if constexpr (dop_looped<G>())
+        DopLane<G>::step_loop(L, y, cf, h, p.mu, p.dir, k, yh, e5, e3);
+      else
+        DopLane<G>::step(L, y, cf, h, p.mu, p.dir, k.v, yh, e5, e3);
       double err_norm;
       {
         double s5[NC], s3[NC];

@@ -100,8 +100,10 @@ int launch(hg::DopParams p, int device, int* counter, cudaStream_t s) {
   // launches without dense samples run the kernel built without that path
   // (fewer registers), as the handle entry point does
   auto kern = p.m >= 2 ? hg::dop853_kernel<G, true> : hg::dop853_kernel<G, false>;
+  constexpr size_t smem = hg::dop_smem_bytes<G>(kBlock);
+  static_assert(smem <= 48 * 1024, "");
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, 0) != cudaSuccess || per_sm < 1) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     per_sm = 1;
   }
@@ -115,7 +117,7 @@ int launch(hg::DopParams p, int device, int* counter, cudaStream_t s) {
     if (cudaMemsetAsync(counter, 0, sizeof(int), s) != cudaSuccess) return HG_ERR_CUDA;
     p.next_traj = counter;
   }
-  kern<<<grid, kBlock, 0, s>>>(p);
+  kern<<<grid, kBlock, smem, s>>>(p);
   return cudaGetLastError() == cudaSuccess ? HG_OK : HG_ERR_CUDA;
 }
 

@@ -279,8 +279,14 @@ struct PairStmHalf {
 // One warp's part of a fixed-step propagation (rk.py:531-588): loads its
 // components, steps through the nodes, writes rows 0, out_every, ...
 // Returns whether its components stayed finite.
+// `sm`: this warp's pair_fixed_doubles<ORDER>(NC) of shared memory (stage
+// derivatives, the step's products).
+template <int ORDER>
+__host__ __device__ constexpr int pair_fixed_doubles(int nc) {
+  return FixedTab<ORDER>::S * nc * 32 + stage_nnz<FixedTab<ORDER>>();
+}
 template <int ORDER, class LT>
-__device__ __forceinline__ bool pair_fixed_run(const LT& L, const FixedParams& p, int traj, bool writes) {
+__device__ __forceinline__ bool pair_fixed_run(const LT& L, const FixedParams& p, int traj, bool writes, double* sm) {
   constexpr int NC = LT::NC;
   double y[NC];
 #pragma unroll
@@ -291,12 +297,13 @@ __device__ __forceinline__ bool pair_fixed_run(const LT& L, const FixedParams& p
   }
   const long long row = 42LL * p.ld_out;
   bool finite = true;
-  WarpCoef<ORDER> cf(threadIdx.x & 31);
+  const StageMem<NC> k{sm + (threadIdx.x & 31)};
+  TableCoef<FixedTab<ORDER>, 32, 1> cf{sm + FixedTab<ORDER>::S * NC * 32, (int)(threadIdx.x & 31), 0xFFFFFFFFu};
   for (int idx = 0; idx < p.n - 1; ++idx) {
     const double h = p.t_vals[idx + 1] - p.t_vals[idx];
     cf.set_step(h);
     double yn[NC];
-    rk_fixed_step<ORDER>(L, y, cf, p.mu, p.dir, yn);
+    rk_fixed_step_loop<ORDER>(L, y, cf, p.mu, p.dir, k, yn);
 #pragma unroll
     for (int r = 0; r < NC; ++r) {
       y[r] = yn[r];
@@ -312,12 +319,18 @@ __device__ __forceinline__ bool pair_fixed_run(const LT& L, const FixedParams& p
   return finite;
 }
 
+template <int ORDER>
+__host__ __device__ constexpr size_t pair_fixed_smem(int block) {
+  return (size_t)(block / 64) * (pair_fixed_doubles<ORDER>(1) + pair_fixed_doubles<ORDER>(6)) * sizeof(double);
+}
+
 // Blocks of 2P warps (P = blockDim.x / 64 pairs): warps 0..P-1 are the state
 // warps of pairs 0..P-1, warps P..2P-1 their STM warps, so each warp of a
 // four-warp block lands on its own sub-partition.
 template <int ORDER>
 __global__ void __launch_bounds__(128) fixed_rk_pair_kernel(FixedParams p) {
   __shared__ PairLink links[2];
+  extern __shared__ double sm_step[];  // pair_fixed_smem<ORDER>(blockDim.x)
   const int w = threadIdx.x >> 5;
   const int npairs = blockDim.x >> 6;
   const int pair = w % npairs;
@@ -349,7 +362,7 @@ __global__ void __launch_bounds__(128) fixed_rk_pair_kernel(FixedParams p) {
       L.link = lk;
       L.seq = 0;
       L.broken = false;
-      finite = pair_fixed_run<ORDER>(L, p, tc, valid && pl.role < 6);
+      finite = pair_fixed_run<ORDER>(L, p, tc, valid && pl.role < 6, sm_step + pair * pair_fixed_doubles<ORDER>(1));
       broken = L.broken;
       finite = __all_sync(pl.gmask, finite);
     } else {
@@ -362,7 +375,8 @@ __global__ void __launch_bounds__(128) fixed_rk_pair_kernel(FixedParams p) {
       L.link = lk;
       L.seq = 0;
       L.broken = false;
-      finite = pair_fixed_run<ORDER>(L, p, tc, valid && pl.role < 6);
+      finite = pair_fixed_run<ORDER>(L, p, tc, valid && pl.role < 6,
+                                     sm_step + npairs * pair_fixed_doubles<ORDER>(1) + pair * pair_fixed_doubles<ORDER>(6));
       broken = L.broken;
       finite = __all_sync(pl.gmask, finite);
       if (pl.role == 0) lk->fin[pl.t] = finite ? 1 : 0;
@@ -385,8 +399,13 @@ __global__ void __launch_bounds__(128) fixed_rk_pair_kernel(FixedParams p) {
 // six warps share an SM's FP64 unit.  The Hessian ring's "empty" barriers
 // take both STM warps' arrivals.
 template <int ORDER>
+__host__ __device__ constexpr size_t trio_fixed_smem() {
+  return (size_t)(pair_fixed_doubles<ORDER>(1) + 2 * pair_fixed_doubles<ORDER>(3)) * sizeof(double);
+}
+template <int ORDER>
 __global__ void __launch_bounds__(96) fixed_rk_trio_kernel(FixedParams p) {
   __shared__ PairLink link;
+  extern __shared__ double sm_step[];  // trio_fixed_smem<ORDER>()
   __shared__ int fin_half[kPairTraj][2];
   const int w = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -416,7 +435,7 @@ __global__ void __launch_bounds__(96) fixed_rk_trio_kernel(FixedParams p) {
       L.link = &link;
       L.seq = 0;
       L.broken = false;
-      finite = pair_fixed_run<ORDER>(L, p, tc, valid && pl.role < 6);
+      finite = pair_fixed_run<ORDER>(L, p, tc, valid && pl.role < 6, sm_step);
       broken = L.broken;
       finite = __all_sync(pl.gmask, finite);
     } else {
@@ -429,7 +448,8 @@ __global__ void __launch_bounds__(96) fixed_rk_trio_kernel(FixedParams p) {
       L.link = &link;
       L.seq = 0;
       L.broken = false;
-      finite = pair_fixed_run<ORDER>(L, p, tc, valid && pl.role < 6);
+      finite = pair_fixed_run<ORDER>(L, p, tc, valid && pl.role < 6,
+                                     sm_step + pair_fixed_doubles<ORDER>(1) + (w - 1) * pair_fixed_doubles<ORDER>(3));
       broken = L.broken;
       finite = __all_sync(pl.gmask, finite);
       if (pl.role == 0) fin_half[tg][hg & 1] = finite ? 1 : 0;
@@ -490,14 +510,23 @@ __device__ __forceinline__ void pair_exchange(const LT& L, PairGather* gx, unsig
   flag_all = (va[42] != 0.0 && va[43] != 0.0 && va[44] != 0.0) ? 1.0 : 0.0;
 }
 
+// Shared memory of a warp: stage derivatives, then its groups' products.
+__host__ __device__ constexpr int pair_dop_doubles(int nc) { return 13 * nc * 32 + stage_nnz<DopTab>() * kPairTraj; }
+__host__ __device__ constexpr size_t pair_dop_smem(int block) {
+  return (size_t)(block / 64) * (pair_dop_doubles(1) + pair_dop_doubles(6)) * sizeof(double);
+}
+__host__ __device__ constexpr size_t trio_dop_smem() {
+  return (size_t)(pair_dop_doubles(1) + 2 * pair_dop_doubles(3)) * sizeof(double);
+}
+
 // One warp's part of the DOP853 propagation of its five trajectories.
 // Decisions that set how many hand-offs a step makes (keep stepping, build a
 // dense cache) are votes over the warp (BLOCK = false: both warps of a pair
 // hold the same trajectories) or over the block (BLOCK = true: the three
 // warps of a trio hold different subsets).  Returns its broken flag.
 template <bool BLOCK, class LT>
-__device__ __forceinline__ bool pair_dop_run(const LT& L, const DopParams& p, PairGather* gx, const double* coef_tab,
-                                             int traj, bool valid, bool writes) {
+__device__ __forceinline__ bool pair_dop_run(const LT& L, const DopParams& p, PairGather* gx, double* sm, int traj,
+                                             bool valid, bool writes) {
   auto vote_any = [](bool v) -> bool {
     if constexpr (BLOCK)
       return __syncthreads_or(v ? 1 : 0) != 0;
@@ -511,8 +540,11 @@ __device__ __forceinline__ bool pair_dop_run(const LT& L, const DopParams& p, Pa
   double y[NC];
 #pragma unroll
   for (int r = 0; r < NC; ++r) y[r] = p.y0[(long long)L.comp(r) * p.ld + traj];
-  double k[13][NC];
-  L.rhs(y, p.mu, p.dir, k[0]);
+  const StageMem<NC> k{sm + (threadIdx.x & 31)};
+  double k0[NC];
+  L.rhs(y, p.mu, p.dir, k0);
+#pragma unroll
+  for (int d = 0; d < NC; ++d) k[0][d] = k0[d];
   unsigned gseq = 0;
   double h;
   {
@@ -521,7 +553,7 @@ __device__ __forceinline__ bool pair_dop_run(const LT& L, const DopParams& p, Pa
     for (int d = 0; d < NC; ++d) {
       const double scale0 = p.atol + p.rtol * fabs(y[d]);
       a[d] = y[d] / scale0;
-      b[d] = k[0][d] / scale0;
+      b[d] = k0[d] / scale0;
     }
     double da, db, unused;
     pair_exchange(L, gx, gseq, a, b, 0.0, da, db, unused);
@@ -539,7 +571,8 @@ __device__ __forceinline__ bool pair_dop_run(const LT& L, const DopParams& p, Pa
   auto sample_t = [&](int q) -> double { return q == p.m - 1 ? tmax : (double)q * step_ls + t0; };
   // integrators/rk.py loop test (t - t_end) * direction < 0, direction +1
   bool live = running && hg_lt0(t - tmax);
-  DopGroupCoef<6> cf(coef_tab, L.role % 6, L.base, L.gmask);
+  // (the shadow lanes of group 4 write their role's entries again)
+  TableCoef<DopTab, 6, kPairTraj> cf{sm + 13 * NC * 32 + L.base / 6, L.role % 6, L.gmask};
   while (vote_any(live)) {
     bool go = live;
     if (go && (long long)(acc + rej) >= p.max_steps) {
@@ -554,7 +587,7 @@ __device__ __forceinline__ bool pair_dop_run(const LT& L, const DopParams& p, Pa
     }
     double yh[NC], e5[NC], e3[NC];
     cf.set_step(hh);
-    DopLaneT<LT>::step(L, y, cf, hh, p.mu, p.dir, k, yh, e5, e3);
+    DopLaneT<LT>::step_loop(L, y, cf, hh, p.mu, p.dir, k, yh, e5, e3);
     double s5[NC], s3[NC];
     bool fin = true;
 #pragma unroll
@@ -655,8 +688,7 @@ __device__ __forceinline__ bool pair_dop_run(const LT& L, const DopParams& p, Pa
 static __global__ void __launch_bounds__(128) dop853_pair_kernel(DopParams p) {
   __shared__ PairLink links[2];
   __shared__ PairGather gathers[2];
-  __shared__ double coef_tab[dop_nnz()];
-  dop_coef_table_init(coef_tab);
+  extern __shared__ double sm_step[];  // pair_dop_smem(blockDim.x)
   const int w = threadIdx.x >> 5;
   const int npairs = blockDim.x >> 6;
   const int pair = w % npairs;
@@ -693,7 +725,7 @@ static __global__ void __launch_bounds__(128) dop853_pair_kernel(DopParams p) {
       L.link = lk;
       L.seq = 0;
       L.broken = false;
-      broken = pair_dop_run<false>(L, p, gx, coef_tab, tc, valid, valid && pl.role < 6);
+      broken = pair_dop_run<false>(L, p, gx, sm_step + pair * pair_dop_doubles(1), tc, valid, valid && pl.role < 6);
     } else {
       PairStm L;
       L.col = pl.role < 6 ? pl.role : 5;
@@ -704,7 +736,8 @@ static __global__ void __launch_bounds__(128) dop853_pair_kernel(DopParams p) {
       L.link = lk;
       L.seq = 0;
       L.broken = false;
-      broken = pair_dop_run<false>(L, p, gx, coef_tab, tc, valid, valid && pl.role < 6);
+      broken = pair_dop_run<false>(L, p, gx, sm_step + npairs * pair_dop_doubles(1) + pair * pair_dop_doubles(6), tc,
+                                   valid, valid && pl.role < 6);
       if (broken && lane == 0) lk->broken = 1;
     }
   }
@@ -721,8 +754,7 @@ static __global__ void __launch_bounds__(128) dop853_pair_kernel(DopParams p) {
 static __global__ void __launch_bounds__(96) dop853_trio_kernel(DopParams p) {
   __shared__ PairLink link;
   __shared__ PairGather gather;
-  __shared__ double coef_tab[dop_nnz()];
-  dop_coef_table_init(coef_tab);
+  extern __shared__ double sm_step[];  // trio_dop_smem()
   const int w = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   if (threadIdx.x < (int)kPairSlots) {
@@ -754,7 +786,7 @@ static __global__ void __launch_bounds__(96) dop853_trio_kernel(DopParams p) {
       L.link = &link;
       L.seq = 0;
       L.broken = false;
-      broken = pair_dop_run<true>(L, p, &gather, coef_tab, tc, valid, valid && pl.role < 6);
+      broken = pair_dop_run<true>(L, p, &gather, sm_step, tc, valid, valid && pl.role < 6);
     } else {
       PairStmHalf L;
       L.t = tg;
@@ -765,7 +797,8 @@ static __global__ void __launch_bounds__(96) dop853_trio_kernel(DopParams p) {
       L.link = &link;
       L.seq = 0;
       L.broken = false;
-      broken = pair_dop_run<true>(L, p, &gather, coef_tab, tc, valid, valid && pl.role < 6);
+      broken = pair_dop_run<true>(L, p, &gather, sm_step + pair_dop_doubles(1) + (w - 1) * pair_dop_doubles(3), tc, valid,
+                                  valid && pl.role < 6);
       if (broken && lane == 0) link.broken = 1;
     }
   }

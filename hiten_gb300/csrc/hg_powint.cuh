@@ -1,0 +1,108 @@
+// Correctly rounded x^y for the step-size controller's exponents on the
+// integer pipes.
+//
+// hg_pow's logarithm and exponential (double-double, hg_crmath.cuh) are about
+// 70 FP64 instructions each, 64 cycles apart for a warp alone: a tenth of a
+// one-lane DOP853 step and a quarter of a six-lane one.  Here log2(x), its
+// product with y and the power of two are 64-bit fixed-point numbers:
+//   log2 x = e + L_j + log2(1 + z), 1 + z = m r_j exact (m the significand,
+//     r_j a 17-bit reciprocal of its upper ten bits), 0 <= z < 2^-9.9, a
+//     degree-5 polynomial; error below 6 units of 2^-64;
+//   T = y (e + f): y is exact in 64 fractional bits, at most 1/8; error
+//     below 0.5 + 6/8 < 1.3 units of 2^-64;
+//   2^T = 2^n E_j 2^t, t < 2^-10, a degree-5 polynomial: R in [2^63, 2^64)
+//     with an error below 0.5 (E_j) + 0.5 (last shift) + 1.3 ln 2 + 0.1 <
+//     2.1 units.
+// R's upper 53 bits, rounded, are the correctly rounded power unless R lies
+// within those 2.1 units of a rounding boundary; then (one power in 340) `ok`
+// is cleared and the caller takes the double-double form.
+#pragma once
+
+#include "hg_exact.cuh"
+#include "hg_powint_tables.h"
+
+#if defined(__CUDACC__)
+__device__ static const uint32_t hg_d_pi_r[1024] = HG_PI_R_INIT;
+__device__ static const unsigned long long hg_d_pi_l[1024] = HG_PI_L_INIT;
+__device__ static const unsigned long long hg_d_pi_e[1024] = HG_PI_E_INIT;
+#endif
+#if defined(__CUDA_ARCH__)
+#define HG_PI_TAB(name, i) __ldg(&hg_d_pi_##name[i])
+#else
+static const uint32_t hg_h_pi_r[1024] = HG_PI_R_INIT;
+static const unsigned long long hg_h_pi_l[1024] = HG_PI_L_INIT;
+static const unsigned long long hg_h_pi_e[1024] = HG_PI_E_INIT;
+#define HG_PI_TAB(name, i) (hg_h_pi_##name[i])
+#endif
+
+HG_XHD uint32_t hgp_mulhi(uint32_t a, uint32_t b) {
+#if defined(__CUDA_ARCH__)
+  return __umulhi(a, b);
+#else
+  return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
+HG_XHD uint64_t hgp_mulhi64(uint64_t a, uint64_t b) {
+#if defined(__CUDA_ARCH__)
+  return __umul64hi(a, b);
+#else
+  return (uint64_t)(((unsigned __int128)a * b) >> 64);
+#endif
+}
+
+// log2(x) = (field - 1023) + f 2^-64 for normal x > 0 (`ok`).
+struct HgLog2 {
+  uint32_t field;
+  uint64_t f;
+  bool ok;
+};
+
+HG_XHD HgLog2 hgp_log2(double x) {
+  HgLog2 r;
+  const uint32_t hi = hgx_hi(x), lo = hgx_lo(x);
+  r.ok = hi - 0x00100000u < 0x7FE00000u;  // positive, normal, finite
+  r.field = hi >> 20;
+  const uint32_t j = (hi >> 10) & 1023u;
+  const uint32_t rj = HG_PI_TAB(r, j);
+  // m r_j - 1 in units of 2^-68, shifted to units of 2^-73 (below 2^63.1)
+  const uint64_t Z = ((uint64_t)lo * rj + ((uint64_t)(((hi & 0xFFFFFu) | 0x100000u) * rj) << 32)) << 5;
+  const uint32_t zh = (uint32_t)(Z >> 32);
+  const uint32_t t = HG_PI_A4 - hgp_mulhi(zh, HG_PI_A5);          // a4 - a5 z, 2^-24
+  const uint32_t h = HG_PI_A3 - hgp_mulhi(zh, t);                 // a3 - z (..), 2^-33
+  const uint64_t s = HG_PI_A2 - (((uint64_t)zh * h) >> 10);       // a2 - z (..), 2^-64
+  const uint64_t w = HG_PI_A1 - (hgp_mulhi64(Z, s) >> 10);        // (a1 - z (..)) / 2, 2^-64
+  r.f = HG_PI_TAB(l, j) + ((hgp_mulhi64(Z, w) + 128u) >> 8);
+  return r;
+}
+
+// RN(x^y) or RN(x^-y) (`neg`) from log2 x; Y = y 2^64, 0 < y <= 1/8 a double.
+HG_XHD double hgp_exp(const HgLog2& g, uint64_t Y, bool neg, bool& ok) {
+  // T = y (field - 1023 + f): 32 integer and 64 fractional bits
+  const uint64_t p0 = (uint64_t)g.field * (uint32_t)Y;
+  const uint64_t p1 = (uint64_t)g.field * (uint32_t)(Y >> 32) + (p0 >> 32);
+  const uint64_t k1 = 1023ull * (uint32_t)(Y >> 32) + ((1023ull * (uint32_t)Y) >> 32);
+  const uint64_t a = (p1 << 32) | (uint32_t)p0, k = (k1 << 32) | (uint32_t)(1023u * (uint32_t)Y);
+  const uint64_t b = hgp_mulhi64(g.f, Y);
+  uint64_t T = a - k;
+  uint32_t n = (uint32_t)(p1 >> 32) - (uint32_t)(k1 >> 32) - (a < k ? 1u : 0u);
+  T += b;
+  n += T < b ? 1u : 0u;
+  if (neg) {  // 2^96 - T, the complement: one unit of 2^-64 less, on the side of the truncation
+    T = ~T;
+    n = ~n;
+  }
+  const uint32_t j = (uint32_t)(T >> 54);
+  const uint64_t tq = T << 10;  // t, 2^-74
+  const uint32_t th = (uint32_t)(tq >> 32);
+  const uint32_t h3 = HG_PI_B3 + hgp_mulhi(th, HG_PI_B4 + hgp_mulhi(th, HG_PI_B5));  // b3 + t (b4 + t b5), 2^-36
+  const uint64_t h2 = HG_PI_B2 + (((uint64_t)th * h3) >> 12);                         // 2^-66
+  const uint64_t h1 = HG_PI_B1 + (hgp_mulhi64(tq, h2) >> 12);                         // 2^-64
+  const uint64_t E = HG_PI_TAB(e, j);
+  const uint64_t R = E + ((hgp_mulhi64(E, hgp_mulhi64(tq, h1)) + 512u) >> 10);        // 2^-63
+  // upper 53 bits, rounded; the boundary (lower bits 1024) at least three
+  // units away, and R not past 2^64 (t within an error of the next power)
+  const uint64_t q = ((R >> 10) + 1u) >> 1;
+  ok = g.ok && (((uint32_t)R + 1024u + 3u) & 2047u) >= 6u && (int64_t)R < 0;
+  const uint64_t bits = q + ((uint64_t)(n + 1022u) << 52);
+  return hgx_make((uint32_t)(bits >> 32), (uint32_t)bits);
+}

@@ -226,9 +226,9 @@ __global__ void collect_kernel(int C, int dim, int hits, const int* list, const 
 }
 
 template <class K>
-int resident_blocks(K kern, int block, int sms) {
+int resident_blocks(K kern, int block, int sms, size_t smem = 0) {
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, 0) != cudaSuccess || per_sm < 1) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     per_sm = 1;
   }
@@ -240,11 +240,11 @@ template <int G>
 cudaError_t segment(hg::DopParams p, int live, int sms, cudaStream_t s) {
   const int tpb = hg::Layout<G>::TPW;
   const int need = (live + tpb - 1) / tpb;
-  const int cap = resident_blocks(hg::dop853_kernel<G, false>, 32, sms);
+  const int cap = resident_blocks(hg::dop853_kernel<G, false>, 32, sms, hg::dop_smem_bytes<G>(32));
   const int grid = need < cap ? need : cap;
   if (grid < 1) return cudaSuccess;
   p.stride = grid * tpb;
-  hg::dop853_kernel<G, false><<<grid, 32, 0, s>>>(p);
+  hg::dop853_kernel<G, false><<<grid, 32, hg::dop_smem_bytes<G>(32), s>>>(p);
   return cudaGetLastError();
 }
 

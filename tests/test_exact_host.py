@@ -3,6 +3,7 @@
 their admitted error, are IEEE's wherever they do not hand the value back; and
 they hand back few."""
 import os
+import platform
 import subprocess
 
 import pytest
@@ -21,3 +22,19 @@ def test_integer_sqrt_and_quotient_match_ieee(tmp_path, seed):
     # handed back: |fr| within 2^-13 (quotient), 4e-4 (root) of a half, two sides each
     assert rq > 100000 and rq - rqo < 1.5 * 2 * 2.0 ** -13 * rq + 50
     assert rs > 100000 and rs - rso < 1.5 * 2 * 4e-4 * rs + 50
+
+
+def test_integer_powers_match_quad(tmp_path):
+    """The step-size controller's powers on the integer pipes
+    (csrc/hg_powint.cuh) are the correctly rounded ones wherever they do not
+    hand the value back (one in 340: six of the 2048 patterns below the
+    rounded bits)."""
+    exe = str(tmp_path / "powint_check")
+    cmd = ["g++", "-O2", "-std=gnu++17", "-ffp-contract=off", "-I" + os.path.join(REPO, "hiten_gb300", "csrc"),
+           os.path.join(REPO, "tests", "native", "powint_check.cpp"), "-o", exe]
+    if platform.machine() not in ("aarch64", "arm64"):
+        cmd.append("-lquadmath")
+    subprocess.check_call(cmd)
+    n, wrong, rnd, ok = map(int, subprocess.check_output([exe, "200000"]).decode().split())
+    assert n > 1_000_000 and wrong == 0
+    assert rnd > 1_000_000 and rnd - ok < 1.5 * 6 / 2048 * rnd
