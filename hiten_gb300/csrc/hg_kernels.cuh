@@ -223,7 +223,7 @@ __device__ __forceinline__ Hess hessian_split(const LT& L, int job, double x, do
   const double ys = L.from(sq, 1);
   const double zs = L.from(sq, 4);
   const double rr = ((b2 ? t2s : t1s) + ys) + zs;
-  const double den = hg_pow15_or_25(rr, k == 2);  // r^3 (jobs 0, 1) or r^5 (job 2) of the lane's primary
+  const double den = hg_power_of_r2(rr, k == 2);  // r^3 (jobs 0, 1) or r^5 (job 2) of the lane's primary
   const double mt = sq;  // jobs 2 and 5
   const double num[2] = {k == 1 ? y : m, k == 0 ? tt : (k == 1 ? z : mt)};
   double quo[2];

@@ -1,7 +1,7 @@
-// Correctly rounded x^y for the step-size controller's exponents on the
-// integer pipes.
+// Correctly rounded powers on the integer pipes: x^y for the step-size
+// controller's exponents, and x^1.5, x^2.5 of the variational equations.
 //
-// hg_pow's logarithm and exponential (double-double, hg_crmath.cuh) are about
+// The controller.  hg_pow's logarithm and exponential (double-double, hg_crmath.cuh) are about
 // 70 FP64 instructions each, 64 cycles apart for a warp alone: a tenth of a
 // one-lane DOP853 step and a quarter of a six-lane one.  Here log2(x), its
 // product with y and the power of two are 64-bit fixed-point numbers:
@@ -106,3 +106,49 @@ HG_XHD double hgp_exp(const HgLog2& g, uint64_t Y, bool neg, bool& ok) {
   const uint64_t bits = q + ((uint64_t)(n + 1022u) << 52);
   return hgx_make((uint32_t)(bits >> 32), (uint32_t)bits);
 }
+
+// RN(x^1.5), or RN(x^2.5) when want25; y as for hgx_sqrt.  With x = m 2^e and
+// sqrt(x) = s 2^k (1 <= m, s < 2), the significand is that of m s or m^2 s:
+//   W: m in 64 bits (exact), or m^2's upper 64 (off by at most 1, centred);
+//   S: s in 64 bits from the root's 53 and its remainder (off by at most
+//     2048 * 3.4e-4 + 0.5 < 1.2);
+//   R = W S / 2^64 normalised to [2^63, 2^64): off by at most 2 (1.2 + 0.5) =
+//     3.4 units (x^1.5), 2 (1.2 + 1 + 0.5) = 5.4 (x^2.5).
+// Closer than that to a rounding boundary (one value in 256 and in 170) `ok`
+// is cleared.
+HG_XHD double hgp_pow15_or_25(double x, float y, bool want25, bool& ok) {
+  uint64_t S_raw;
+  float fr;
+  hgx_sqrt_parts(x, y, S_raw, fr);
+  const uint32_t hi = hgx_hi(x), lo = hgx_lo(x);
+  const uint64_t S = ((S_raw - ((uint64_t)HGX_OFFSET << 32)) << 11) +
+                     (uint64_t)(int64_t)(int32_t)(hgx_fbits(fmaf(fr, 2048.0f, HGX_M2)) - HGX_M2_BITS);
+  const uint64_t m = ((uint64_t)(((hi & 0xFFFFFu) | 0x100000u) << 11 | lo >> 21) << 32) | (lo << 11);
+  uint64_t mm = hgp_mulhi64(m, m);
+  const uint32_t sm = (uint32_t)(~mm >> 63);  // m^2 < 2
+  mm = (mm << sm) + sm;
+  const uint64_t W = want25 ? mm : m;
+  uint64_t R = hgp_mulhi64(W, S);
+  const uint32_t sr = (uint32_t)(~R >> 63);
+  R = (R << sr) + sr;
+  // exponent: e + floor(e / 2), or 2 e + floor(e / 2), plus one for every
+  // product that reached 2
+  const int32_t e = (int32_t)(hi >> 20) - 1023;
+  const int32_t ex = e + (e >> 1) + (want25 ? e + 1 - (int32_t)sm : 0) + 1 - (int32_t)sr;
+  const uint64_t q = ((R >> 10) + 1u) >> 1;
+  const uint32_t w = want25 ? 6u : 4u;
+  // |e| < 100: the powers stay far from the ends of the range
+  ok = (hi - (923u << 20)) < (200u << 20) && (((uint32_t)R + 1024u + w) & 2047u) >= 2u * w;
+  const uint64_t bits = q + ((uint64_t)(uint32_t)(ex + 1022) << 52);
+  return hgx_make((uint32_t)(bits >> 32), (uint32_t)bits);
+}
+
+#if defined(__CUDACC__)
+// x^1.5 or x^2.5, with the double-double form behind it
+__device__ __forceinline__ double hg_power_of_r2(double x, bool want25) {
+  bool ok;
+  double p = hgp_pow15_or_25(x, hgx_rsqrt_approx(hgx_sqrt_arg(x)), want25, ok);
+  if (!ok) p = hg_pow15_or_25(x, want25);
+  return p;
+}
+#endif

@@ -2,8 +2,8 @@
 // quad-precision pow rounded once: the controller's three exponents on random
 // errors over the whole range, every table entry's first and last significand,
 // and significands next to a power of two.  A power whose `ok` is set must be
-// the correctly rounded one.  Prints
-// "<powers> <wrong> <random powers> <of them ok>".
+// the correctly rounded one.  The same for x^1.5 and x^2.5.  Prints
+// "<powers> <wrong> <random powers> <of them ok> <random x^1.5, x^2.5> <of them ok>".
 #include <stdio.h>
 #include <stdlib.h>
 
@@ -26,11 +26,25 @@ static uint64_t next64() {  // splitmix64
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
   return z ^ (z >> 31);
 }
-static long powers, wrong, random_powers, random_ok;
+static long powers, wrong, random_powers, random_ok, roots, root_ok;
 static double make(uint64_t bits) {
   double x;
   memcpy(&x, &bits, 8);
   return x;
+}
+// x^1.5 and x^2.5 with the FP32 estimate k ulps from the best
+static void check_r2(uint64_t bits, int k) {
+  const double x = make(bits);
+  const double t = 1.0 / sqrt((double)hgx_sqrt_arg(x));
+  float y = hgx_float(hgx_fbits((float)t) + (uint32_t)k);
+  if (fabs(y / t - 1.0) > 1.2783e-7) y = (float)t;
+  for (bool want25 : {false, true}) {
+    bool ok;
+    const double p = hgp_pow15_or_25(x, y, want25, ok);
+    ++roots;
+    root_ok += ok;
+    if (ok && p != (double)QPOW((q_t)x, (q_t)(want25 ? 2.5 : 1.5))) ++wrong;
+  }
 }
 static void check(uint64_t bits, bool random) {
   double x;
@@ -60,8 +74,23 @@ int main(int argc, char** argv) {
     check(((983 + r % 50) << 52) | m, true);
     check(((983 + r % 50) << 52) | ((r >> 40) & 1 ? (1ull << 52) - 1 - (m & 15) : (m & 15)), false);
   }
+  long edges = 0, edge_ok = 0;
+  for (long i = 0; i < n; ++i) {
+    const uint64_t r = next64(), m = next64() >> 12;
+    check_r2(((983 + r % 80) << 52) | m, (int)((r >> 32) % 5) - 2);
+    edges -= roots, edge_ok -= root_ok;
+    check_r2(((983 + r % 80) << 52) | ((r >> 40) & 1 ? (1ull << 52) - 1 - (m & 255) : (m & 255)), 0);
+    edges += roots, edge_ok += root_ok;
+  }
+  roots -= edges, root_ok -= edge_ok;
+  for (double x : {0.0, -1.0, 5e-324, 1e-40, 1e40, (double)INFINITY, (double)NAN})
+    for (bool want25 : {false, true}) {
+      bool ok;
+      hgp_pow15_or_25(x, 1.0f, want25, ok);
+      if (ok) ++wrong;
+    }
   for (double x : {0.0, -1.0, 5e-324, 1e-310, (double)INFINITY, (double)NAN})
     if (hgp_log2(x).ok) ++wrong;
-  printf("%ld %ld %ld %ld\n", powers, wrong, random_powers, random_ok);
+  printf("%ld %ld %ld %ld %ld %ld\n", powers, wrong, random_powers, random_ok, roots, root_ok);
   return 0;
 }

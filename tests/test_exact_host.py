@@ -35,6 +35,8 @@ def test_integer_powers_match_quad(tmp_path):
     if platform.machine() not in ("aarch64", "arm64"):
         cmd.append("-lquadmath")
     subprocess.check_call(cmd)
-    n, wrong, rnd, ok = map(int, subprocess.check_output([exe, "200000"]).decode().split())
+    n, wrong, rnd, ok, rts, rok = map(int, subprocess.check_output([exe, "200000"]).decode().split())
     assert n > 1_000_000 and wrong == 0
     assert rnd > 1_000_000 and rnd - ok < 1.5 * 6 / 2048 * rnd
+    # x^1.5 hands back 8 of 2048 patterns, x^2.5 twelve
+    assert rts == 400_000 and rts - rok < 1.5 * 10 / 2048 * rts
