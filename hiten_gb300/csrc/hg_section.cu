@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include "hg_exact.cuh"
 #include "hitengpu.h"
 
 namespace {
@@ -332,36 +333,92 @@ __global__ void __launch_bounds__(128) section_kernel(SecParams p) {
 // (np.sqrt((x + mu)**2 + y**2 + z**2), numpy squares being x*x) and the
 // maximum relative Jacobi-constant drift of common/energy.py:26-74
 // (numba: squares x*x, **0.5 of a positive number = the correctly rounded
-// square root).  One thread per trajectory.
-__global__ void __launch_bounds__(128) filters_kernel(int N, int m, const double* samples, long long ld, double mu,
-                                                       double* min_r1, double* min_r2, double* max_rel_e) {
+// square root).
+//
+// One thread per trajectory and chunk of samples; chunks so many that the
+// device is full (a manifold has tens to thousands of trajectories of thousands
+// of samples: one thread for all samples of each left 12 of 152 SMs busy and
+// took 16.3 ms for 1600 x 4713, 0.49 ms here).  Bound: the FP64 unit, 27
+// instructions a sample (0.33 ms); the two roots and quotients are on the integer pipes
+// (hg_exact.cuh), and what is monotone is taken once per trajectory: the root
+// of the least squared distance, the quotient of the largest |C - C0|.
+// The chunks' results meet in the outputs as integers: non-negative doubles
+// order like their bit patterns, in which a NaN is above everything.
+struct FilterSample {
+  double q1, q2;  // squared distances to the primaries
+  double C;       // Jacobi constant
+};
+
+__device__ __forceinline__ FilterSample filter_sample(const double* s, long long ld, double mu, double mu1) {
+  FilterSample r;
+  const double x = s[0], y = s[ld], z = s[2 * ld], vx = s[3 * ld], vy = s[4 * ld], vz = s[5 * ld];
+  const double a = x + mu, b = (x - 1.0) + mu, f = x - mu1;
+  const double yy = y * y, zz = z * z;
+  r.q1 = (a * a + yy) + zz;
+  r.q2 = (b * b + yy) + zz;
+  const double r1 = hg_sqrt(r.q1), r2 = hg_sqrt((f * f + yy) + zz);
+  r.C = ((x * x + yy) + 2.0 * (hg_div(mu1, r1) + hg_div(mu, r2))) - ((vx * vx + vy * vy) + vz * vz);
+  return r;
+}
+
+__device__ __forceinline__ unsigned long long pattern(double v) { return (unsigned long long)__double_as_longlong(v); }
+
+// The reference's running minimum keeps a first NaN and passes over later
+// ones; its running maximum starts at 0 and passes over NaN.
+__device__ __forceinline__ void filter_finish(const FilterSample& first, unsigned long long q1, unsigned long long q2,
+                                              unsigned long long e, double* min_r1, double* min_r2,
+                                              double* max_rel_e) {
+  const double absC0 = fabs(first.C), d = __longlong_as_double((long long)e);
+  const double rel = absC0 > 1e-14 ? d / absC0 : d;
+  *min_r1 = first.q1 != first.q1 ? first.q1 : sqrt(__longlong_as_double((long long)q1));
+  *min_r2 = first.q2 != first.q2 ? first.q2 : sqrt(__longlong_as_double((long long)q2));
+  *max_rel_e = rel > 0.0 ? rel : 0.0;
+}
+
+constexpr int kFilterBlock = 64;
+constexpr int kFilterChunk = 16;  // least samples per chunk: each one also forms C of sample 0
+
+// ONE: a single chunk, finished here; else the outputs hold bit patterns.
+template <bool ONE>
+__global__ void __launch_bounds__(kFilterBlock) filters_kernel(int N, int m, int chunk, const double* samples,
+                                                               long long ld, double mu, double* min_r1,
+                                                               double* min_r2, double* max_rel_e) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const double mu1 = 1.0 - mu, mu2 = mu;
-  double C0 = 0.0, absC0 = 0.0, emax = 0.0, m1 = 0.0, m2 = 0.0;
-  for (int q = 0; q < m; ++q) {
-    const double* s = samples + (long long)q * 6 * ld + i;
-    const double x = s[0], y = s[ld], z = s[2 * ld], vx = s[3 * ld], vy = s[4 * ld], vz = s[5 * ld];
-    const double a = x + mu, b = (x - 1.0) + mu;
-    const double d1 = sqrt((a * a + y * y) + z * z);
-    const double d2 = sqrt((b * b + y * y) + z * z);
-    m1 = (q == 0 || d1 < m1) ? d1 : m1;
-    m2 = (q == 0 || d2 < m2) ? d2 : m2;
-    const double e = x + mu2, f = x - mu1;
-    const double r1 = sqrt((e * e + y * y) + z * z);
-    const double r2 = sqrt((f * f + y * y) + z * z);
-    const double C = ((x * x + y * y) + 2.0 * (mu1 / r1 + mu2 / r2)) - ((vx * vx + vy * vy) + vz * vz);
-    if (q == 0) {
-      C0 = C;
-      absC0 = fabs(C0);
-    } else {
-      const double rel = absC0 > 1e-14 ? fabs(C - C0) / absC0 : fabs(C - C0);
-      if (rel > emax) emax = rel;
-    }
+  const double mu1 = 1.0 - mu;
+  const FilterSample first = filter_sample(samples + i, ld, mu, mu1);
+  unsigned long long q1 = pattern(first.q1), q2 = pattern(first.q2), e = 0;
+  const int lo = max(1, (int)blockIdx.y * chunk), hi = min(m, ((int)blockIdx.y + 1) * chunk);
+  for (int q = lo; q < hi; ++q) {
+    const FilterSample s = filter_sample(samples + (long long)q * 6 * ld + i, ld, mu, mu1);
+    const unsigned long long p1 = pattern(s.q1), p2 = pattern(s.q2), d = pattern(fabs(s.C - first.C));
+    q1 = p1 < q1 ? p1 : q1;
+    q2 = p2 < q2 ? p2 : q2;
+    e = d > e && d <= 0x7FF0000000000000ull ? d : e;
   }
-  min_r1[i] = m1;
-  min_r2[i] = m2;
-  max_rel_e[i] = emax;
+  if constexpr (ONE) {
+    filter_finish(first, q1, q2, e, min_r1 + i, min_r2 + i, max_rel_e + i);
+  } else {
+    atomicMin((unsigned long long*)min_r1 + i, q1);
+    atomicMin((unsigned long long*)min_r2 + i, q2);
+    atomicMax((unsigned long long*)max_rel_e + i, e);
+  }
+}
+
+__global__ void filters_init_kernel(int N, double* min_r1, double* min_r2, double* max_rel_e) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  ((unsigned long long*)min_r1)[i] = ((unsigned long long*)min_r2)[i] = ~0ull;
+  ((unsigned long long*)max_rel_e)[i] = 0ull;
+}
+
+__global__ void filters_finish_kernel(int N, const double* samples, long long ld, double mu, double* min_r1,
+                                      double* min_r2, double* max_rel_e) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  const FilterSample first = filter_sample(samples + i, ld, mu, 1.0 - mu);
+  filter_finish(first, pattern(min_r1[i]), pattern(min_r2[i]), pattern(max_rel_e[i]), min_r1 + i, min_r2 + i,
+                max_rel_e + i);
 }
 
 }  // namespace
@@ -371,9 +428,26 @@ extern "C" int hg_trajectory_filters(int N, int m, const double* samples, long l
   if (N < 0 || m < 1 || ld < N) return HG_ERR_ARGS;
   if (N > 0 && (!samples || !min_r1 || !min_r2 || !max_rel_energy)) return HG_ERR_ARGS;
   if (N == 0) return HG_OK;
-  const int block = 128;
-  filters_kernel<<<(N + block - 1) / block, block, 0, (cudaStream_t)stream>>>(N, m, samples, ld, mu, min_r1, min_r2,
-                                                                              max_rel_energy);
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return HG_ERR_CUDA;
+  const cudaStream_t st = (cudaStream_t)stream;
+  // chunks: about 24 warps per SM in all
+  const int bx = (N + kFilterBlock - 1) / kFilterBlock;
+  const int most = (m + kFilterChunk - 1) / kFilterChunk;
+  const long long want = (12LL * sms + bx - 1) / bx;
+  const int parts = (int)(want < most ? want : most);
+  const int chunk = (m + parts - 1) / parts;
+  if (parts <= 1) {
+    filters_kernel<true><<<bx, kFilterBlock, 0, st>>>(N, m, m, samples, ld, mu, min_r1, min_r2, max_rel_energy);
+  } else {
+    const int bi = (N + 127) / 128;
+    filters_init_kernel<<<bi, 128, 0, st>>>(N, min_r1, min_r2, max_rel_energy);
+    filters_kernel<false><<<dim3((unsigned)bx, (unsigned)((m + chunk - 1) / chunk)), kFilterBlock, 0, st>>>(
+        N, m, chunk, samples, ld, mu, min_r1, min_r2, max_rel_energy);
+    filters_finish_kernel<<<bi, 128, 0, st>>>(N, samples, ld, mu, min_r1, min_r2, max_rel_energy);
+  }
   return cudaGetLastError() == cudaSuccess ? HG_OK : HG_ERR_CUDA;
 }
 
