@@ -69,13 +69,15 @@ def config(n_gpus):
             "parallelism": f"replicas x{n_gpus}", "l2": "flushed between timed steps (256 MiB write)"}
 
 
-def sched_lanes(n_live, warp_slots):
+def sched_lanes(n_live, warp_slots, sms=152):
     """Lanes per trajectory the scheduled DOP853 driver gives a segment of
-    n_live trajectories: the least of lat(G) x max(1, warps / warp_slots)
-    (the same rule as the library's)."""
+    n_live trajectories (the same rule as the library's: the layout of least
+    time per step, its latency up to the warps an SM's FP64 unit serves and
+    growing with the load beyond)."""
     best, best_cost = 1, None
-    for g, per_warp, lat in ((1, 32, 1.0), (2, 16, 0.622), (6, 5, 0.400)):
-        cost = lat * max(1.0, -(-n_live // per_warp) / warp_slots)
+    for g, per_warp, lat, cap in ((6, 5, 0.354, 5.42), (2, 16, 0.644, 5.07), (1, 32, 1.0, 4.27)):
+        load = -(-n_live // per_warp) / (cap * sms + 0.5 * (warp_slots - 3.0 * sms))
+        cost = lat ** 4 * (1.0 + load ** 4)
         if best_cost is None or cost < best_cost:
             best, best_cost = g, cost
     return best
@@ -91,7 +93,7 @@ def dominant_launch(run_segment, plan, n, sm_count, stream, reps=3):
     import torch
     if not plan.get("scheduled"):
         return None
-    g = plan.get("lanes_d6") or sched_lanes(n, plan.get("sm_capacity", 3.0) * sm_count)
+    g = plan.get("lanes_d6") or sched_lanes(n, plan.get("sm_capacity", 3.0) * sm_count, sm_count)
     seg = int(plan.get("seg_steps", 16))
     run_segment(g, seg)  # warm
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)

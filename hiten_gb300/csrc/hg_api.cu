@@ -5,6 +5,8 @@
 // (sized by hg_reserve / hg_reserve_correct, or grown on first use); every
 // allocation is counted (HG_COUNTER_ALLOCATIONS).
 #include <cuda_runtime.h>
+
+#include <algorithm>
 #include <stdarg.h>
 #include <stdio.h>
 #include <string.h>
@@ -72,7 +74,41 @@ hg::Dir make_dir(int dim, int fwd, int flip_lo, int flip_hi) {
   return d;
 }
 
+// Allow a kernel more dynamic shared memory than a launch gets unasked.
+template <class K>
+bool allow_smem(K kernel, size_t bytes) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
+}
+
+// Lanes per 6-dim trajectory when the caller did not choose.
+int auto_lanes_d6(const hg_handle* h, int N) {
+  return hg_internal::lanes_d6(N, h->sm_count, 0.1 * h->sm_capacity_x10);
+}
+
 // Blocks default to one warp: small batches then spread over all SMs.
+
+// 6-dim fixed step without an event.
+template <int ORDER, int G>
+int launch_fixed_d6(hg_handle* h, const hg::FixedParams& p, cudaStream_t s) {
+  const int tpb = (h->block / 32) * hg::Layout<G>::TPW;
+  const int grid = (p.N + tpb - 1) / tpb;
+  if (grid < 1) return HG_OK;
+  const size_t smem = hg::fixed_smem_bytes<ORDER, G>(h->block);
+  if (smem > 48 * 1024 && !allow_smem(hg::fixed_rk_d6_kernel<ORDER, G>, smem))
+    return fail(h, HG_ERR_CUDA, "shared memory");
+  hg::fixed_rk_d6_kernel<ORDER, G><<<grid, h->block, smem, s>>>(p);
+  return check_launch(h, "fixed_rk_d6_kernel");
+}
+
+template <int ORDER>
+int launch_fixed_d6(hg_handle* h, const hg::FixedParams& p, cudaStream_t s) {
+  const int g = auto_lanes_d6(h, p.N);
+  if (g == 6) return launch_fixed_d6<ORDER, 6>(h, p, s);
+  if (g == 2) return launch_fixed_d6<ORDER, 2>(h, p, s);
+  return launch_fixed_d6<ORDER, 1>(h, p, s);
+}
 
 template <int ORDER, int G>
 int launch_fixed(hg_handle* h, const hg::FixedParams& p, cudaStream_t s) {
@@ -81,6 +117,8 @@ int launch_fixed(hg_handle* h, const hg::FixedParams& p, cudaStream_t s) {
   if (grid > 0) {
     if constexpr (G == 14) {
       hg::fixed_rk_kernel<ORDER, G><<<grid, h->block, 0, s>>>(p);
+    } else if constexpr (G == 1) {
+      hg::fixed_rk_event_kernel<ORDER, G><<<grid, h->block, 0, s>>>(p);
     } else {
       if (p.ev_index >= 0)
         hg::fixed_rk_event_kernel<ORDER, G><<<grid, h->block, 0, s>>>(p);
@@ -91,47 +129,25 @@ int launch_fixed(hg_handle* h, const hg::FixedParams& p, cudaStream_t s) {
   return check_launch(h, "fixed_rk_kernel");
 }
 
-// Lanes per 42-dim trajectory: 7 (an STM column per lane) or 14 (half a
-// column per lane: half the stage work per lane, twice the warps).  Unless
-// fixed by tuning, the one with the least time per step, where a warp's step
-// takes lat(G) (G = 14: 0.65 of G = 7) while its SM holds at most three
-// warps' FP64 demand, beyond which warps share the SM's FP64 unit.  With
-// `pair` the paired-warp layout (12 lanes on two warps, five trajectories
-// per pair, lat 0.6: RK8 on GB300, 125 ms against 214 ms for G = 7 over 3000
-// steps of 512 states) competes too.
-int lanes_d42(const hg_handle* h, int n, bool pair = false, double pair_lat = 0.0) {
-  if (h->lanes_d42 != 0) return ((h->lanes_d42 == 12 || h->lanes_d42 == 18) && !pair) ? 7 : h->lanes_d42;
+// Lanes per 42-dim trajectory of a run with an event or in segments: 7 (an STM
+// column per lane) or 14 (half a column per lane: half the stage work per
+// lane, twice the warps).  Unless fixed by tuning, the one with the least time
+// per step, where a warp's step takes lat(G) (G = 14: 0.65 of G = 7) while its
+// SM holds at most three warps' FP64 demand, beyond which warps share the
+// SM's FP64 unit.
+int lanes_d42(const hg_handle* h, int n) {
+  if (h->lanes_d42 != 0) return (h->lanes_d42 == 12 || h->lanes_d42 == 18) ? 7 : h->lanes_d42;
   const double cap = 0.1 * h->sm_capacity_x10 * h->sm_count;
   const double w7 = (double)((n + 3) / 4), w14 = (double)((n + 1) / 2);
-  const double wp = 2.0 * (double)((n + hg::kPairTraj - 1) / hg::kPairTraj);
   const double c7 = 1.0 * (w7 > cap ? w7 / cap : 1.0);
   const double c14 = 0.65 * (w14 > cap ? w14 / cap : 1.0);
-  const double cp = pair_lat * (wp > cap ? wp / cap : 1.0);
-  if (pair && pair_lat > 0.0 && cp < c7 && cp < c14) return 12;
   return c14 < c7 ? 14 : 7;
 }
 
-// Per-step latency of the paired-warp layout relative to G = 7 (0: not
-// chosen automatically).
-constexpr double kPairLatFixed = 0.6;
-// Event-free single-pass DOP853 on 42 components: the three-warp layout
-// (state warp + two half-column STM warps) while its warps fit about three
-// per SM (3 N / 5 <= 3 x SMs), the pair above -- measured for the corrector's
-// STM legs (ms: 64 orbits trio 1.60, pair 1.81, G = 14 1.91, G = 7 2.43; 512
-// orbits 1.68 / 1.88 / 1.95 / 2.53; 2048 orbits 2.91 / 2.66 / 3.42 / 2.97)
-// and one trajectory with 2000 dense samples (7.4 / 10.6 / 9.3 / 15.0).
-int lanes_d42_dop_free(const hg_handle* h, int n) {
+// Event-free single-pass 42-dim runs, fixed-step and DOP853.
+int lanes_d42_free(const hg_handle* h, int n) {
   if (h->lanes_d42 != 0) return h->lanes_d42;
-  const double cap = 0.1 * h->sm_capacity_x10 * h->sm_count;
-  return 3.0 * ((n + hg::kPairTraj - 1) / hg::kPairTraj) <= cap ? 18 : 12;
-}
-
-// Allow a kernel more dynamic shared memory than a launch gets unasked.
-template <class K>
-bool allow_smem(K kernel, size_t bytes) {
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess) return true;
-  cudaGetLastError();
-  return false;
+  return hg_internal::lanes_d42_free(n, h->sm_count, 0.1 * h->sm_capacity_x10);
 }
 
 // Paired-warp DOP853 launch (42-dim, no event, single pass): blocks of one
@@ -208,12 +224,17 @@ int fixed_common(hg_handle* h, double mu, int order, int dim, int N, const doubl
 }
 
 int fixed_dispatch(hg_handle* h, int order, int dim, const hg::FixedParams& p, cudaStream_t s) {
+  if (dim == 6 && p.ev_index < 0) {
+    if (order == 4) return launch_fixed_d6<4>(h, p, s);
+    if (order == 6) return launch_fixed_d6<6>(h, p, s);
+    return launch_fixed_d6<8>(h, p, s);
+  }
   if (dim == 6) {
     if (order == 4) return launch_fixed<4, 1>(h, p, s);
     if (order == 6) return launch_fixed<6, 1>(h, p, s);
     return launch_fixed<8, 1>(h, p, s);
   }
-  const int g42 = p.ev_index < 0 ? lanes_d42(h, p.N, true, kPairLatFixed) : 7;
+  const int g42 = p.ev_index < 0 ? lanes_d42_free(h, p.N) : 7;
   if (g42 == 18) {
     if (order == 4) return launch_fixed_trio<4>(h, p, s);
     if (order == 6) return launch_fixed_trio<6>(h, p, s);
@@ -317,9 +338,8 @@ template <int G, class K>
 Shape dop_shape(const hg_handle* h, K kernel) {
   Shape sh{h->block, hg::dop_smem_bytes<G>(h->block), 1};
   if (h->spread && h->smem_per_sm > 0) {
-    const size_t half = (size_t)(h->smem_per_sm / 2 + 1024);
     sh.block = 128;
-    sh.smem = hg::dop_smem_bytes<G>(128) > half ? hg::dop_smem_bytes<G>(128) : half;
+    sh.smem = std::max(hg::dop_smem_bytes<G>(128), (size_t)(h->smem_per_sm / 2 + 1024));
   }
   if (sh.smem > 32 * 1024 &&  // with the static part above the 48 KB a launch gets unasked
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem) != cudaSuccess) {
@@ -359,18 +379,6 @@ int launch_dop853(hg_handle* h, hg::DopParams p, cudaStream_t s) {
   }
   kern<<<grid, kBlock, sh.smem, s>>>(p);
   return check_launch(h, "dop853_kernel");
-}
-
-// Lanes per 6-dim DOP853 trajectory when the caller did not choose: the
-// largest group whose warps still fit four per SM, about what an SM's FP64
-// unit serves at each warp's full rate (the longest trajectory sets the time
-// and its per-step latency falls with the group size), single lanes once even
-// those oversubscribe.
-int auto_lanes_d6(const hg_handle* h, int N) {
-  const long long smsp = 4LL * h->sm_count;
-  if ((N + 4LL) / 5 <= smsp) return 6;
-  if ((N + 15LL) / 16 <= smsp) return 2;
-  return 1;
 }
 
 __global__ void seg_init_kernel(int N, int* list, int* count, int* status) {
@@ -470,32 +478,6 @@ int launch_dop853_seg(hg_handle* h, hg::DopParams p, const SegWs& w, int seg_ste
       return fail(h, HG_ERR_CUDA, "memcpy");
   }
   return HG_OK;
-}
-
-// Layout of the next segment of a 6-dim batch with n_live trajectories
-// left: the group size with the least time per step.  One warp's step takes
-// lat(G) while its SM is not saturated (measured on GB300 for the longest
-// manifold trajectory: 75.4, 46.9 and 30.2 us for G = 1, 2, 6); an SM's FP64
-// unit serves about three such warps at full speed (two run as fast as one,
-// four lose ~13 %), beyond which they share it.
-int sched_lanes_d6(const hg_handle* h, int n_live) {
-  if (h->lanes_d6 != 0) return h->lanes_d6;
-  const double smsp = 0.1 * h->sm_capacity_x10 * h->sm_count;
-  const int gs[3] = {1, 2, 6};
-  const int tpw[3] = {32, 16, 5};
-  const double lat[3] = {1.0, 0.622, 0.400};
-  int best = 0;
-  double best_cost = 0.0;
-  for (int i = 0; i < 3; ++i) {
-    const double warps = (double)((n_live + tpw[i] - 1) / tpw[i]);
-    const double load = warps / smsp;
-    const double cost = lat[i] * (load > 1.0 ? load : 1.0);
-    if (i == 0 || cost < best_cost) {
-      best = i;
-      best_cost = cost;
-    }
-  }
-  return gs[best];
 }
 
 __global__ void fp64_probe_kernel(double* out, int iters, double a, double b) {
@@ -707,7 +689,7 @@ int hg_propagate_dop853(hg_handle* h, double mu, int dim, int N, const double* y
     else
       rc2 = launch_dop853<1>(h, p, s);
   } else {
-    const int g = p.ev_index < 0 ? lanes_d42_dop_free(h, N) : lanes_d42(h, N);
+    const int g = p.ev_index < 0 ? lanes_d42_free(h, N) : lanes_d42(h, N);
     if (g == 12 && p.ev_index < 0)
       rc2 = launch_dop853_pair(h, p, s);
     else if (g == 18 && p.ev_index < 0)
@@ -804,7 +786,7 @@ int hg_propagate_dop853_scheduled(hg_handle* h, double mu, int dim, int N, const
   int n_live = N, a = 0;
   for (long long it = 0; it < max_iter && n_live > 0; ++it) {
     if (dim == 6) {
-      const int g = sched_lanes_d6(h, n_live);
+      const int g = h->lanes_d6 != 0 ? h->lanes_d6 : auto_lanes_d6(h, n_live);
       if (g == 6)
         rc = launch_segment<6>(h, p, w, (int)seg, a, n_live, s);
       else if (g == 2)

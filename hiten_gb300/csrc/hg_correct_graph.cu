@@ -702,18 +702,15 @@ void stm_leg(const Ws& w, double mu, const hg_newton_opts& o, int sms, cudaStrea
 
 int lanes_d6(int n, int sms, int tuned) {
   if (tuned == 1 || tuned == 2 || tuned == 6) return tuned;
-  const long long smsp = 4LL * sms;
-  if ((n + 4LL) / 5 <= smsp) return 6;
-  if ((n + 15LL) / 16 <= smsp) return 2;
-  return 1;
+  return hg_internal::lanes_d6(n, sms, 3.0);
 }
 
-// STM leg layout: the handle's tuning, else the three-warp layout while its
-// warps fit about three per SM (3 N / 5 <= 3 x SMs) and the paired warps above
-// (the host driver's rule for event-free 42-dim legs).
+// STM leg layout: the handle's tuning, else the rule of event-free 42-dim runs
+// for two thirds of the orbits: they leave as they converge (2048 orbits: trio
+// 18.4 ms, pair 19.6; 4096: 30.5 and 26.3).
 int lanes_d42(int tuned, int n, int sms) {
   if (tuned == 7 || tuned == 14 || tuned == 12 || tuned == 18) return tuned;
-  return 3LL * ((n + hg::kPairTraj - 1) / hg::kPairTraj) <= 3LL * sms ? 18 : 12;
+  return hg_internal::lanes_d42_free(2LL * n / 3, sms, 3.0);
 }
 
 void event_leg_any(int g, const Ws& w, double mu, const hg_newton_opts& o, int sms, cudaStream_t s, int* n) {

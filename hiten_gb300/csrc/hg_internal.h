@@ -22,4 +22,47 @@ void count_launches(hg_handle* h, long long n);
 int device_of(const hg_handle* h);
 int tuning(const hg_handle* h, int key);
 
+// Lanes per 6-dim trajectory for a launch that steps n of them side by side:
+// the group size with the least time per step.  A layout's step takes its
+// latency while its warps fit an SM's FP64 unit (`cap` of them; in between the
+// fourth-power mean of both fits the measurements within 6 %) and grows with
+// the warps per SM beyond.  Measured on GB300 (us per DOP853 step, 152 SMs):
+//   n        1     3040   4864   7296   9728   14592  19456  29184  48640
+//   1 lane   55.4  55.9   56.0   55.9   56.0   56.1   60.9   81.2   131
+//   2 lanes  32.7  36.0   36.0   36.0   38.9   45.9   56.9   83.8   138
+//   6 lanes  18.4  20.4   26.2   35.2   46.1   80.7   93.0   133    212
+// sm_capacity (the tuning value, 3 by default) moves the capacities.
+inline int lanes_d6(long long n, int sms, double sm_capacity) {
+  const int gs[3] = {6, 2, 1};
+  const long long per_warp[3] = {5, 16, 32};
+  const double lat[3] = {0.354, 0.644, 1.0}, cap[3] = {5.42, 5.07, 4.27};
+  int best = 1;
+  double best_cost = 0.0;
+  for (int i = 0; i < 3; ++i) {
+    const double warps = (double)((n + per_warp[i] - 1) / per_warp[i]);
+    const double slots = (cap[i] + 0.5 * (sm_capacity - 3.0)) * sms;
+    const double l2 = (warps / slots) * (warps / slots), lat2 = lat[i] * lat[i];
+    const double cost = lat2 * lat2 * (1.0 + l2 * l2);
+    if (i == 0 || cost < best_cost) {
+      best = gs[i];
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
+// Layout of an event-free single-pass 42-dim run of n trajectories: three warps
+// per five of them (18) while an SM holds at most two such groups, warp pairs
+// (12) beyond.  Measured on GB300 (us per step; G = 7 and 14 are behind at
+// every size):
+//   n              760    1000   1500   2048   4096   8192
+//   RK8, trio      28.5   35.2   35.2   50.3   100    178
+//   RK8, pair      40.5   40.9   41.0   45.8   82.9   165
+//   DOP853, trio   38.7   45.4   45.4   61.9   139    217
+//   DOP853, pair   52.2   52.8   52.9   58.2   98.6   195
+inline int lanes_d42_free(long long n, int sms, double sm_capacity) {
+  const double groups = (double)((n + 4) / 5);
+  return groups <= 2.0 * (sm_capacity / 3.0) * sms ? 18 : 12;
+}
+
 }  // namespace hg_internal

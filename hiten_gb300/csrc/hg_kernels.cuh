@@ -963,79 +963,6 @@ struct InlineCoef {
   }
 };
 
-// Position of a_ij (i >= 1, j < i, nonzero) in the list of the tableau's
-// nonzero A entries by rows, followed by the nonzero B entries (b_j at
-// fixed_flat(S, j)); -1 for a zero entry.
-template <int ORDER>
-__host__ __device__ constexpr int fixed_flat(int i, int j) {
-  using T = FixedTab<ORDER>;
-  int q = 0;
-  for (int r = 1; r < T::S; ++r)
-    for (int c = 0; c < r; ++c) {
-      if (T::a(r, c) != 0.0) {
-        if (r == i && c == j) return q;
-        ++q;
-      }
-    }
-  for (int c = 0; c < T::S; ++c) {
-    if (T::b(c) != 0.0) {
-      if (i == T::S && c == j) return q;
-      ++q;
-    }
-  }
-  return -1;
-}
-
-// The same products spread over a warp whose lanes all step with the same h
-// (fixed-step runs): lane l forms the products of list positions l, l + 32
-// and l + 64 (three FP64 multiplies per step instead of one per entry) and
-// each stage fetches its coefficients by shuffle.  Bit-identical: every
-// product is the same h * a.  All 32 lanes must be present.
-template <int ORDER>
-struct WarpCoef {
-  static_assert(fixed_flat<ORDER>(FixedTab<ORDER>::S, FixedTab<ORDER>::S) < 0, "");
-  double base[3];  // this lane's tableau entries
-  double v[3];     // this lane's products for the current step
-  __device__ __forceinline__ explicit WarpCoef(int lane) {
-    using T = FixedTab<ORDER>;
-    base[0] = base[1] = base[2] = 0.0;
-    static_for<T::S>([&](auto ic) {
-      constexpr int i = decltype(ic)::value;
-      static_for<i>([&](auto jc) {
-        constexpr int j = decltype(jc)::value;
-        if constexpr (T::a(i, j) != 0.0) {
-          constexpr int q = fixed_flat<ORDER>(i, j);
-          static_assert(q >= 0 && q < 96, "");
-          if (lane == q % 32) base[q / 32] = T::a(i, j);
-        }
-      });
-    });
-    static_for<T::S>([&](auto jc) {
-      constexpr int j = decltype(jc)::value;
-      if constexpr (T::b(j) != 0.0) {
-        constexpr int q = fixed_flat<ORDER>(T::S, j);
-        static_assert(q >= 0 && q < 96, "");
-        if (lane == q % 32) base[q / 32] = T::b(j);
-      }
-    });
-  }
-  __device__ __forceinline__ void set_step(double h) {
-    v[0] = h * base[0];
-    v[1] = h * base[1];
-    v[2] = h * base[2];
-  }
-  template <int I, int J>
-  __device__ __forceinline__ double a() const {
-    constexpr int q = fixed_flat<ORDER>(I, J);
-    return __shfl_sync(0xFFFFFFFFu, v[q / 32], q % 32);
-  }
-  template <int J>
-  __device__ __forceinline__ double b() const {
-    constexpr int q = fixed_flat<ORDER>(FixedTab<ORDER>::S, J);
-    return __shfl_sync(0xFFFFFFFFu, v[q / 32], q % 32);
-  }
-};
-
 template <int ORDER, class LT, class CF>
 __device__ __forceinline__ void rk_fixed_step(const LT& L, const double (&y)[LT::NC], const CF& cf, double mu,
                                               const Dir& dir, double (&yn)[LT::NC]) {
@@ -1229,6 +1156,82 @@ __global__ void __launch_bounds__(128) fixed_rk_event_kernel(FixedParams p) {
   }
 }
 
+// 6-dim fixed step without an event, one, two or six lanes per trajectory
+// (hg_internal::lanes_d6 chooses).  The step size is the launch's, so the
+// products h a_ij are formed once per step by the whole warp; lanes beyond the
+// batch, and lanes 30 and 31 of the six-lane layout, repeat a neighbour's
+// trajectory and write nothing.  Bound by the latency of a step's chain up to
+// about 3000 trajectories, by the FP64 unit beyond 20000.  Against one lane
+// per trajectory at every size (us per step): RK4 777 states 13.7 -> 4.9, 9000
+// 13.7 -> 7.5, 40000 34.1 -> 19.7; RK8 61.3 -> 18.2, 61.3 -> 34.0, 161 -> 109.
+template <int ORDER, int G>
+__host__ __device__ constexpr int fixed_warp_doubles() {
+  return FixedTab<ORDER>::S * Layout<G>::NC * 32 + stage_nnz<FixedTab<ORDER>>();
+}
+template <int ORDER, int G>
+__host__ __device__ constexpr size_t fixed_smem_bytes(int block) {
+  return (size_t)(block / 32) * fixed_warp_doubles<ORDER, G>() * sizeof(double);
+}
+template <int ORDER, int G>
+__global__ void __launch_bounds__(128) fixed_rk_d6_kernel(FixedParams p) {
+  using T = FixedTab<ORDER>;
+  constexpr int NC = Layout<G>::NC, TPW = Layout<G>::TPW;
+  extern __shared__ double sm_step[];  // fixed_smem_bytes<ORDER, G>(blockDim.x)
+  const int lane = threadIdx.x & 31;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if ((long long)warp * TPW >= p.N) return;  // the whole warp
+  Layout<G> L;
+  const int g = lane / G < TPW ? lane / G : TPW - 1;
+  if constexpr (G == 1) {
+    L.role = 6;
+  } else {
+    L.role = lane % G;
+    L.base = g * G;
+    L.gmask = G == 6 ? (g < 4 ? 0x3Fu << L.base : 0xFF000000u) : 0x3u << L.base;
+  }
+  const int traj = warp * TPW + g < p.N ? warp * TPW + g : p.N - 1;
+  const bool writes = lane < TPW * G && warp * TPW + g < p.N;
+  double* const sm = sm_step + (threadIdx.x >> 5) * fixed_warp_doubles<ORDER, G>();
+  const StageMem<NC> k{sm + lane};
+  TableCoef<T, 32, 1> cf{sm + T::S * NC * 32, lane, 0xFFFFFFFFu};
+  double y[NC];
+#pragma unroll
+  for (int r = 0; r < NC; ++r) y[r] = p.y0[(long long)L.comp(r) * p.ld_in + traj];
+  if (writes) {
+#pragma unroll
+    for (int r = 0; r < NC; ++r) p.out[(long long)L.comp(r) * p.ld_out + traj] = y[r];
+  }
+  const long long row = 6 * p.ld_out;
+  bool finite = true;
+  double t = p.t_vals[0];
+  int left = p.out_every;
+  double* o = p.out + row;
+  for (int idx = 1; idx < p.n; ++idx) {
+    const double t1 = p.t_vals[idx];
+    cf.set_step(t1 - t);
+    t = t1;
+    double yn[NC];
+    rk_fixed_step_loop<ORDER>(L, y, cf, p.mu, p.dir, k, yn);
+#pragma unroll
+    for (int r = 0; r < NC; ++r) {
+      y[r] = yn[r];
+      finite = finite && finite_bits(yn[r]);
+    }
+    if (--left == 0) {
+      left = p.out_every;
+      if (writes) {
+#pragma unroll
+        for (int r = 0; r < NC; ++r) o[(long long)L.comp(r) * p.ld_out + traj] = y[r];
+      }
+      o += row;
+    }
+  }
+  if (p.status) {
+    if constexpr (G > 1) finite = __all_sync(L.gmask, finite);
+    if (writes && (G == 1 || L.role == 0)) p.status[traj] = finite ? HG_OK : HG_NONFINITE;
+  }
+}
+
 template <int ORDER, int G>
 __global__ void __launch_bounds__(128) fixed_rk_kernel(FixedParams p) {
   constexpr int NC = Layout<G>::NC;
@@ -1236,10 +1239,7 @@ __global__ void __launch_bounds__(128) fixed_rk_kernel(FixedParams p) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   Layout<G> L;
   int traj;
-  if constexpr (G == 1) {
-    L.role = 6;
-    traj = warp * 32 + lane;
-  } else if constexpr (G == 14) {
+  if constexpr (G == 14) {
     if (lane >= 28) return;
     const int g = lane / 14;
     L.role = lane % 14;
@@ -1278,11 +1278,9 @@ __global__ void __launch_bounds__(128) fixed_rk_kernel(FixedParams p) {
     }
   }
   if (p.status) {
-    if constexpr (G > 1) {
-      finite = __all_sync(L.gmask, finite);
-      // one lane of the group writes the status
-      if (L.role != (G == 7 ? 6 : 0)) return;
-    }
+    finite = __all_sync(L.gmask, finite);
+    // one lane of the group writes the status
+    if (L.role != (G == 7 ? 6 : 0)) return;
     p.status[traj] = finite ? HG_OK : HG_NONFINITE;
   }
 }

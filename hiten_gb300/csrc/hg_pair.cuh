@@ -512,9 +512,11 @@ __device__ __forceinline__ void pair_exchange(const LT& L, PairGather* gx, unsig
 
 // Shared memory of a warp: stage derivatives, then its groups' products.
 __host__ __device__ constexpr int pair_dop_doubles(int nc) { return 13 * nc * 32 + stage_nnz<DopTab>() * kPairTraj; }
-__host__ __device__ constexpr size_t pair_dop_smem(int block) {
-  return (size_t)(block / 64) * (pair_dop_doubles(1) + pair_dop_doubles(6)) * sizeof(double);
+// A pair's link, gather slots and both warps' parts.
+__host__ __device__ constexpr size_t pair_dop_bytes() {
+  return sizeof(PairLink) + sizeof(PairGather) + (pair_dop_doubles(1) + pair_dop_doubles(6)) * sizeof(double);
 }
+__host__ __device__ constexpr size_t pair_dop_smem(int block) { return (size_t)(block / 64) * pair_dop_bytes(); }
 __host__ __device__ constexpr size_t trio_dop_smem() {
   return (size_t)(pair_dop_doubles(1) + 2 * pair_dop_doubles(3)) * sizeof(double);
 }
@@ -685,15 +687,21 @@ __device__ __forceinline__ bool pair_dop_run(const LT& L, const DopParams& p, Pa
 }
 
 // Blocks of one or two pairs, laid out as fixed_rk_pair_kernel's.
-static __global__ void __launch_bounds__(128) dop853_pair_kernel(DopParams p) {
-  __shared__ PairLink links[2];
-  __shared__ PairGather gathers[2];
-  extern __shared__ double sm_step[];  // pair_dop_smem(blockDim.x)
+// Six blocks of one pair per SM: 168 registers a thread (the dense cache of an
+// STM column, built once or never per trajectory, spills 100 bytes) and 36.5 KB
+// of shared memory; at the 255 registers taken unasked four blocks fit, and
+// 4096 trajectories (5.4 groups per SM) took two rounds.
+static __global__ void __launch_bounds__(128, 3) dop853_pair_kernel(DopParams p) {
+  static_assert(sizeof(PairLink) % 8 == 0 && sizeof(PairGather) % 8 == 0, "");
+  extern __shared__ double sm_step[];  // pair_dop_smem(blockDim.x): links, gathers, the warps' parts
   const int w = threadIdx.x >> 5;
   const int npairs = blockDim.x >> 6;
   const int pair = w % npairs;
   const bool stm = w >= npairs;
   const int lane = threadIdx.x & 31;
+  PairLink* const links = (PairLink*)sm_step;
+  PairGather* const gathers = (PairGather*)(links + npairs);
+  double* const sm = (double*)(gathers + npairs);
   PairLink* lk = &links[pair];
   PairGather* gx = &gathers[pair];
   if (threadIdx.x < npairs * (int)kPairSlots) {
@@ -725,7 +733,7 @@ static __global__ void __launch_bounds__(128) dop853_pair_kernel(DopParams p) {
       L.link = lk;
       L.seq = 0;
       L.broken = false;
-      broken = pair_dop_run<false>(L, p, gx, sm_step + pair * pair_dop_doubles(1), tc, valid, valid && pl.role < 6);
+      broken = pair_dop_run<false>(L, p, gx, sm + pair * pair_dop_doubles(1), tc, valid, valid && pl.role < 6);
     } else {
       PairStm L;
       L.col = pl.role < 6 ? pl.role : 5;
@@ -736,7 +744,7 @@ static __global__ void __launch_bounds__(128) dop853_pair_kernel(DopParams p) {
       L.link = lk;
       L.seq = 0;
       L.broken = false;
-      broken = pair_dop_run<false>(L, p, gx, sm_step + npairs * pair_dop_doubles(1) + pair * pair_dop_doubles(6), tc,
+      broken = pair_dop_run<false>(L, p, gx, sm + npairs * pair_dop_doubles(1) + pair * pair_dop_doubles(6), tc,
                                    valid, valid && pl.role < 6);
       if (broken && lane == 0) lk->broken = 1;
     }

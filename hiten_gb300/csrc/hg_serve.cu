@@ -44,6 +44,7 @@
 #include <thread>
 #include <vector>
 
+#include "hg_internal.h"
 #include "hg_kernels.cuh"
 #include "hitengpu.h"
 
@@ -261,25 +262,11 @@ cudaError_t refine(hg::DopParams p, int sms, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// Lanes per trajectory for a segment of n live trajectories: the least
-// lat(G) x max(1, warps / capacity), the host-scheduled driver's rule.
+// Lanes per trajectory for a segment of n live trajectories: the
+// host-scheduled driver's rules.
 int lanes_for(int dim, int n, int sms) {
   const double cap = 3.0 * sms;
-  if (dim == 6) {
-    const int gs[3] = {1, 2, 6}, tpw[3] = {32, 16, 5};
-    const double lat[3] = {1.0, 0.622, 0.400};
-    int best = 0;
-    double bc = 0.0;
-    for (int i = 0; i < 3; ++i) {
-      const double warps = (double)((n + tpw[i] - 1) / tpw[i]);
-      const double c = lat[i] * std::max(1.0, warps / cap);
-      if (i == 0 || c < bc) {
-        best = i;
-        bc = c;
-      }
-    }
-    return gs[best];
-  }
+  if (dim == 6) return hg_internal::lanes_d6(n, sms, 3.0);
   const double w7 = (double)((n + 3) / 4), w14 = (double)((n + 1) / 2);
   const double c7 = std::max(1.0, w7 / cap), c14 = 0.65 * std::max(1.0, w14 / cap);
   return c14 < c7 ? 14 : 7;
