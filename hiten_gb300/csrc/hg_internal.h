@@ -28,9 +28,9 @@ int tuning(const hg_handle* h, int key);
 // fourth-power mean of both fits the measurements within 6 %) and grows with
 // the warps per SM beyond.  Measured on GB300 (us per DOP853 step, 152 SMs):
 //   n        1     3040   4864   7296   9728   14592  19456  29184  48640
-//   1 lane   55.4  55.9   56.0   55.9   56.0   56.1   60.9   81.2   131
-//   2 lanes  32.7  36.0   36.0   36.0   38.9   45.9   56.9   83.8   138
-//   6 lanes  18.4  20.4   26.2   35.2   46.1   80.7   93.0   133    212
+//   1 lane   54.7  55.1   55.1   55.2   55.1   55.0   60.5   80.7   131
+//   2 lanes  31.1  34.4   34.5   34.5   37.3   45.1   57.0   83.5   138
+//   6 lanes  17.3  19.3   25.5   34.6   45.7   70.4   92.7   132    211
 // sm_capacity (the tuning value, 3 by default) moves the capacities.
 inline int lanes_d6(long long n, int sms, double sm_capacity) {
   const int gs[3] = {6, 2, 1};

@@ -87,6 +87,12 @@ struct DopTab {
 // Vector fields
 // ---------------------------------------------------------------------------
 
+// -v when neg: the sign-bit flip IEEE negation is, on the integer pipe (the
+// FP64 pipe is the scarce one).
+__device__ __forceinline__ double neg_if(double v, bool neg) {
+  return __longlong_as_double(__double_as_longlong(v) ^ (neg ? (long long)0x8000000000000000ull : 0ll));
+}
+
 // dynamics/rtbp.py:30-74 (_crtbp_accel), numba lowering of ** (x*x, x*(x*x)).
 // The distances and the six quotients over r1^3 and r2^3 are formed on the
 // FP32 and integer pipes (hg_exact.cuh): the bits of sqrt and `/`, with 31
@@ -94,24 +100,29 @@ struct DopTab {
 __device__ __forceinline__ void rhs6(const double (&s)[6], double mu, double (&d)[6]) {
   const double x = s[0], y = s[1], z = s[2], vx = s[3], vy = s[4];
   const double omu = 1.0 - mu;
+  // What does not need the distances stands before the roots, so that its FP64
+  // instructions run beside their integer sequences.
   const double t1 = x + mu;
   const double yy = y * y;
   const double zz = z * z;
-  const double r1 = hg_sqrt((t1 * t1 + yy) + zz);
+  const double s1 = (t1 * t1 + yy) + zz;
   const double t2 = x - omu;
-  const double r2 = hg_sqrt((t2 * t2 + yy) + zz);
-  const double r1c = r1 * (r1 * r1);
-  const double r2c = r2 * (r2 * r2);
+  const double s2 = (t2 * t2 + yy) + zz;
   const double n1[3] = {omu * t1, omu * y, (-omu) * z};
   const double n2[3] = {mu * ((x - 1.0) + mu), mu * y, mu * z};
+  const double cx = 2.0 * vy + x, cy = -2.0 * vx + y;
+  const double r1 = hg_sqrt(s1);
+  const double r2 = hg_sqrt(s2);
+  const double r1c = r1 * (r1 * r1);
+  const double r2c = r2 * (r2 * r2);
   double q1[3], q2[3];
   hg_quotients(n1, r1c, q1);
   hg_quotients(n2, r2c, q2);
   d[0] = vx;
   d[1] = vy;
   d[2] = s[5];
-  d[3] = ((2.0 * vy + x) - q1[0]) - q2[0];
-  d[4] = ((-2.0 * vx + y) - q1[1]) - q2[1];
+  d[3] = (cx - q1[0]) - q2[0];
+  d[4] = (cy - q1[1]) - q2[1];
   d[5] = q1[2] - q2[2];
 }
 
@@ -161,12 +172,6 @@ __device__ __forceinline__ Hess hessian42(double x, double y, double z, double v
 struct Dir {
   int neg_lo, neg_hi;  // component range whose derivative is negated (fwd=-1)
 };
-
-// -v when neg: the sign-bit flip IEEE negation is, on the integer pipe (the
-// FP64 pipe is the scarce one).
-__device__ __forceinline__ double neg_if(double v, bool neg) {
-  return __longlong_as_double(__double_as_longlong(v) ^ (neg ? (long long)0x8000000000000000ull : 0ll));
-}
 
 template <int G>
 struct Layout;
@@ -425,9 +430,12 @@ struct Layout<2> {
     const double sqo = __shfl_xor_sync(gmask, sq, 1);
     const double yy = r0 ? sq : sqo;
     const double zz = r0 ? sqo : sq;
-    const double r = hg_sqrt((t * t + yy) + zz);
-    const double rc = r * (r * r);
+    // what does not need the distance stands before its root (see rhs6)
+    const double s2 = (t * t + yy) + zz;
     const double n[3] = {mb * ((x + a1) + a2), mb * y, mz * z};
+    const double r = hg_sqrt(s2);
+    const double rc = r * (r * r);
+    const double cor = (r0 ? 2.0 : -2.0) * (r0 ? vy : vx) + (r0 ? x : y);
     double q[3];
     hg_quotients(n, rc, q);
     const double qx = q[0], qy = q[1], qz = q[2];
@@ -439,7 +447,7 @@ struct Layout<2> {
     const double pz = __shfl_xor_sync(gmask, qz, 1);
     const double q1 = r0 ? qx : p;
     const double q2 = r0 ? p : qy;
-    const double acc = (((r0 ? 2.0 : -2.0) * (r0 ? vy : vx) + (r0 ? x : y)) - q1) - q2;
+    const double acc = (cor - q1) - q2;
     const double ax = __shfl_xor_sync(gmask, acc, 1);
     const double az = pz - qz;
     dv[0] = r0 ? vx : ax;
@@ -484,33 +492,35 @@ struct Layout<6> {
     const bool b0 = role < 3;
     const int ax = b0 ? role : role - 3;
     const double omu = 1.0 - mu;
-    const double cb = b0 ? mu : -omu;  // x + mu | x - (1 - mu)
-    const double a1 = b0 ? mu : -1.0;  // x-numerator: (x + a1) + a2
-    const double a2 = b0 ? 0.0 : mu;
-    const double t = x + cb;
-    // the squares t_b^2, y^2, z^2 in one multiply: lane (b, a) squares t_b,
-    // y or z for a = 0, 1, 2, and each lane gathers its primary's three
-    const double w = ax == 0 ? t : (ax == 1 ? y : z);
-    const double sq = w * w;
+    // The chain below is what a step waits for.  A value that leaves the FP64
+    // unit and comes back (a select or a shuffle between two FP64
+    // instructions) costs about 31 cycles more than the next instruction taking
+    // it directly, so selects stand before the arithmetic, with neutral
+    // operands where a lane has nothing to add; and the sums that do not need
+    // the distance stand where the chain waits (1797 -> 1576 cycles per
+    // evaluation, one warp).
+    // lane (b, a): t_b, y or z (+ 0 changes the sign of a zero, then squared)
+    const double e = ax == 0 ? x : (ax == 1 ? y : z);
+    const double t = e + (ax == 0 ? (b0 ? mu : -omu) : 0.0);
+    const double sq = t * t;
+    // x-numerators (x + mu) + 0 and (x - 1) + mu
+    const double nx = (x + (b0 ? mu : -1.0)) + (b0 ? 0.0 : mu);
     const double tt = __shfl_sync(gmask, sq, base + (b0 ? 0 : 3));
     const double yy = __shfl_sync(gmask, sq, base + 1);
     const double zz = __shfl_sync(gmask, sq, base + 2);
-    const double r = hg_sqrt((tt + yy) + zz);
-    const double rc = r * (r * r);
-    const double nx = (x + a1) + a2;
-    const double nb = ax == 0 ? nx : (ax == 1 ? y : z);
+    const double s2 = (tt + yy) + zz;
     const double m = b0 ? (ax == 2 ? -omu : omu) : mu;
-    const double n[1] = {m * nb};
+    const double n[1] = {m * (ax == 0 ? nx : e)};
+    const double r = hg_sqrt(s2);
+    const double rc = r * (r * r);
+    const double cor = (role == 3 ? 2.0 : -2.0) * u + (role == 3 ? x : y);
     double qq[1];
     hg_quotients(n, rc, qq);
-    const double q = qq[0];
-    // first primary's quotient of this lane's axis (lanes 3..5 use it)
-    const double pq = __shfl_sync(gmask, q, base + ax);
-    const double c2 = role == 3 ? 2.0 : -2.0;
-    const double xy = role == 3 ? x : y;
-    const double acc_xy = ((c2 * u + xy) - pq) - q;
-    const double acc_z = pq - q;
-    const double d = role < 3 ? u : (role == 5 ? acc_z : acc_xy);
+    // first primary's quotient of this lane's axis.  Lanes 3 and 4: (cor -
+    // q1) - q2; lane 5: q1z - q2z; lanes 0..2: u (minus zero)
+    const double pq = __shfl_sync(gmask, qq[0], base + ax);
+    const bool xy = role == 3 || role == 4;
+    const double d = ((b0 ? u : (xy ? cor : pq)) - (xy ? pq : 0.0)) - (b0 ? 0.0 : qq[0]);
     dv[0] = neg_if(d, role >= dir.neg_lo && role < dir.neg_hi);
   }
 };
