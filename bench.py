@@ -73,9 +73,10 @@ def sched_lanes(n_live, warp_slots, sms=152):
     """Lanes per trajectory the scheduled DOP853 driver gives a segment of
     n_live trajectories (the same rule as the library's: the layout of least
     time per step, its latency up to the warps an SM's FP64 unit serves and
-    growing with the load beyond)."""
+    growing with the load beyond; among the layouts `lanes_d6` can fix, so 6
+    where the driver gives a trajectory a whole warp)."""
     best, best_cost = 1, None
-    for g, per_warp, lat, cap in ((6, 5, 0.354, 5.42), (2, 16, 0.644, 5.07), (1, 32, 1.0, 4.27)):
+    for g, per_warp, lat, cap in ((6, 5, 0.336, 5.15), (2, 16, 0.625, 5.05), (1, 32, 1.0, 4.35)):
         load = -(-n_live // per_warp) / (cap * sms + 0.5 * (warp_slots - 3.0 * sms))
         cost = lat ** 4 * (1.0 + load ** 4)
         if best_cost is None or cost < best_cost:

@@ -105,7 +105,7 @@ int launch_fixed_d6(hg_handle* h, const hg::FixedParams& p, cudaStream_t s) {
 template <int ORDER>
 int launch_fixed_d6(hg_handle* h, const hg::FixedParams& p, cudaStream_t s) {
   const int g = auto_lanes_d6(h, p.N);
-  if (g == 6) return launch_fixed_d6<ORDER, 6>(h, p, s);
+  if (g == 6 || g == 30) return launch_fixed_d6<ORDER, 6>(h, p, s);
   if (g == 2) return launch_fixed_d6<ORDER, 2>(h, p, s);
   return launch_fixed_d6<ORDER, 1>(h, p, s);
 }
@@ -684,6 +684,8 @@ int hg_propagate_dop853(hg_handle* h, double mu, int dim, int N, const double* y
     if (lanes == 0) lanes = auto_lanes_d6(h, N);
     if (lanes == 6)
       rc2 = launch_dop853<6>(h, p, s);
+    else if (lanes == 30)
+      rc2 = launch_dop853<30>(h, p, s);
     else if (lanes == 2)
       rc2 = launch_dop853<2>(h, p, s);
     else
@@ -740,6 +742,8 @@ int hg_propagate_dop853_segmented(hg_handle* h, double mu, int dim, int N, const
     if (lanes == 0) lanes = auto_lanes_d6(h, N);
     if (lanes == 6)
       rc = launch_dop853_seg<6>(h, p, w, seg_steps, max_segments, resume, s);
+    else if (lanes == 30)
+      rc = launch_dop853_seg<30>(h, p, w, seg_steps, max_segments, resume, s);
     else if (lanes == 2)
       rc = launch_dop853_seg<2>(h, p, w, seg_steps, max_segments, resume, s);
     else
@@ -789,6 +793,8 @@ int hg_propagate_dop853_scheduled(hg_handle* h, double mu, int dim, int N, const
       const int g = h->lanes_d6 != 0 ? h->lanes_d6 : auto_lanes_d6(h, n_live);
       if (g == 6)
         rc = launch_segment<6>(h, p, w, (int)seg, a, n_live, s);
+      else if (g == 30)
+        rc = launch_segment<30>(h, p, w, (int)seg, a, n_live, s);
       else if (g == 2)
         rc = launch_segment<2>(h, p, w, (int)seg, a, n_live, s);
       else

@@ -714,7 +714,9 @@ int lanes_d42(int tuned, int n, int sms) {
 }
 
 void event_leg_any(int g, const Ws& w, double mu, const hg_newton_opts& o, int sms, cudaStream_t s, int* n) {
-  if (g == 6)
+  if (g == 30)
+    event_leg<30>(w, mu, o, sms, s, n);
+  else if (g == 6)
     event_leg<6>(w, mu, o, sms, s, n);
   else if (g == 2)
     event_leg<2>(w, mu, o, sms, s, n);

@@ -23,22 +23,24 @@ int device_of(const hg_handle* h);
 int tuning(const hg_handle* h, int key);
 
 // Lanes per 6-dim trajectory for a launch that steps n of them side by side:
-// the group size with the least time per step.  A layout's step takes its
-// latency while its warps fit an SM's FP64 unit (`cap` of them; in between the
-// fourth-power mean of both fits the measurements within 6 %) and grows with
-// the warps per SM beyond.  Measured on GB300 (us per DOP853 step, 152 SMs):
-//   n        1     3040   4864   7296   9728   14592  19456  29184  48640
-//   1 lane   54.7  55.1   55.1   55.2   55.1   55.0   60.5   80.7   131
-//   2 lanes  31.1  34.4   34.5   34.5   37.3   45.1   57.0   83.5   138
-//   6 lanes  17.3  19.3   25.5   34.6   45.7   70.4   92.7   132    211
+// the layout with the least time per step (30: five six-lane groups on one
+// trajectory, a warp each).  A layout's step takes its latency while its warps
+// fit an SM's FP64 unit (`cap` of them; in between the fourth-power mean of
+// both fits the measurements within 6 %) and grows with the warps per SM
+// beyond.  Measured on GB300 (us per DOP853 step, 152 SMs):
+//   n         1     608    912    1216   3040   4864   7296   9728   14592  19456  29184  48640
+//   1 lane    54.7  55.3   55.0   55.0   55.1   55.1   55.2   55.1   55.0   60.5   80.7   131
+//   2 lanes   31.1  34.4   34.5   34.5   34.4   34.5   34.5   37.3   45.1   57.0   83.5   138
+//   6 lanes   17.3  18.6   18.5   18.6   19.3   25.5   34.6   45.7   70.4   92.7   132    211
+//   30 lanes  15.1  16.1   17.4   21.2   (57 at 2280)
 // sm_capacity (the tuning value, 3 by default) moves the capacities.
 inline int lanes_d6(long long n, int sms, double sm_capacity) {
-  const int gs[3] = {6, 2, 1};
-  const long long per_warp[3] = {5, 16, 32};
-  const double lat[3] = {0.354, 0.644, 1.0}, cap[3] = {5.42, 5.07, 4.27};
+  const int gs[4] = {30, 6, 2, 1};
+  const long long per_warp[4] = {1, 5, 16, 32};
+  const double lat[4] = {0.287, 0.336, 0.625, 1.0}, cap[4] = {6.6, 5.15, 5.05, 4.35};
   int best = 1;
   double best_cost = 0.0;
-  for (int i = 0; i < 3; ++i) {
+  for (int i = 0; i < 4; ++i) {
     const double warps = (double)((n + per_warp[i] - 1) / per_warp[i]);
     const double slots = (cap[i] + 0.5 * (sm_capacity - 3.0)) * sms;
     const double l2 = (warps / slots) * (warps / slots), lat2 = lat[i] * lat[i];

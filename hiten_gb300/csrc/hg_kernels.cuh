@@ -525,6 +525,15 @@ struct Layout<6> {
   }
 };
 
+// G = 30 (6-dim state, one trajectory per warp): five copies of the six-lane
+// group.  All five step the same trajectory with the same instructions; what
+// they share out is the stage sums (step_eager) and the dense samples.
+template <>
+struct Layout<30> : Layout<6> {
+  static constexpr int TPW = 1;
+};
+constexpr unsigned kWarp30 = 0x3FFFFFFFu;  // lanes 30 and 31 idle
+
 // numpy float64 dot order of the host the reference fixtures come from:
 // sequential fused accumulation for n < 16, a 32-element blocked sum plus a
 // fused tail for n = 42.  v is the full vector (identical in every lane).
@@ -709,6 +718,9 @@ struct Gather<6> {
     db = __shfl_sync(L.gmask, s, L.base + 3);
   }
 };
+
+template <>
+struct Gather<30> : Gather<6> {};
 
 // v[r] for a runtime r without dynamic register indexing.
 template <int NC>
@@ -1477,6 +1489,35 @@ struct StageRegs {
   __device__ __forceinline__ const double (&operator[](int j) const)[NC] { return v[j]; }
 };
 
+// The sums of one DOP853 step shared over the five groups of a warp (G = 30):
+// sum T = 5 s + g + 1 belongs to group g, slot s -- T = 1 .. 11 the stage
+// arguments, 12 the step's end, 13 and 14 the error sums err5 and err3.  Entry
+// (s, j, g) of the list is sum T's coefficient of k_j; bit g of used[s][j]
+// tells that it is not zero.
+struct EagerList {
+  double c[3 * 13 * 5];
+  int used[3][13];
+};
+__host__ __device__ constexpr EagerList make_eager_list() {
+  EagerList t{};
+  for (int s = 0; s < 3; ++s)
+    for (int j = 0; j < 13; ++j)
+      for (int g = 0; g < 5; ++g) {
+        const int T = 5 * s + g + 1;
+        double v = 0.0;
+        if (T < DopTab::S)
+          v = j < T ? DopTab::a(T, j) : 0.0;
+        else if (T == DopTab::S)
+          v = j < DopTab::S ? DopTab::b(j) : 0.0;
+        else if (T <= 14)
+          v = T == 13 ? DopTab::e5(j) : DopTab::e3(j);
+        t.c[(s * 13 + j) * 5 + g] = v;
+        if (v != 0.0) t.used[s][j] |= 1 << g;
+      }
+  return t;
+}
+__device__ static const EagerList hg_eager_list = make_eager_list();
+
 template <class LT>
 struct DopLaneT {
   static constexpr int NC = LT::NC;
@@ -1507,6 +1548,38 @@ struct DopLaneT {
       e5[d] = e5[d] * h;
       e3[d] = e3[d] * h;
     }
+  }
+
+  // One attempted step by five groups of six lanes (G = 30).  As soon as k_j
+  // exists every sum that has it takes its term -- each group those of its
+  // own sums, at most three multiplies and adds for all five groups instead
+  // of one per sum -- and the next stage's argument is read from its group.
+  // Every sum has the terms and the order of the other forms.  `tab`: h times
+  // the stage entries of hg_eager_list and the error sums' entries as they
+  // are (EagerCoef::set_step), for this lane's group.
+  __device__ __forceinline__ static void step_eager(const LT& L, const double (&y)[1], const double* tab, double h,
+                                                    double mu, const Dir& dir, double (&k)[13][1], double (&yh)[1],
+                                                    double (&e5)[1], double (&e3)[1]) {
+    constexpr EagerList el = make_eager_list();
+    const int g = L.base / 6;
+    double acc[3] = {y[0], y[0], g < 2 ? y[0] : 0.0};
+    static_for<13>([&](auto jc) {
+      constexpr int j = decltype(jc)::value;
+      constexpr int first = j < 12 ? j / 5 : 2;  // slot of the next stage's sum
+      static_for<3>([&](auto oc) {
+        constexpr int o = decltype(oc)::value;
+        constexpr int sl = o == 0 ? first : (o <= first ? o - 1 : o);
+        constexpr int used = el.used[sl][j];
+        if constexpr (used != 0) {
+          const double sum = acc[sl] + tab[(sl * 13 + j) * 5] * k[j][0];
+          acc[sl] = used == 31 || ((used >> g) & 1) ? sum : acc[sl];
+        }
+        if constexpr (o == 0 && j < 12) yh[0] = __shfl_sync(kWarp30, acc[first], (j % 5) * 6 + L.role);
+      });
+      if constexpr (j < 12) L.rhs(yh, mu, dir, k[j + 1]);
+    });
+    e5[0] = __shfl_sync(kWarp30, acc[2], 12 + L.role) * h;
+    e3[0] = __shfl_sync(kWarp30, acc[2], 18 + L.role) * h;
   }
 
   // One attempted step with the stages as a loop: k[0] on entry, k[1..12] on
@@ -1655,11 +1728,30 @@ __host__ __device__ constexpr bool dop_looped() {
   return G == 1 || G == 2;
 }
 
-// Dynamic shared memory of a dop853_kernel<G> warp in the looped form: stage
-// derivatives, then (G > 1) the step's products.
+// The five groups' coefficients of a step (G = 30), entry (s, j, g) of the
+// warp's table at (s * 13 + j) * 5 + g.
+struct EagerCoef {
+  double* tab;  // the warp's table
+  int lane, g;
+  __device__ __forceinline__ void set_step(double h) {
+    __syncwarp(kWarp30);
+#pragma unroll
+    for (int i = 0; i < 7; ++i) {
+      const int q = lane + 30 * i;
+      // groups 2 and 3 hold the error sums in slot 2
+      const double f = q >= 2 * 65 && q % 5 >= 2 ? 1.0 : h;
+      if (q < 3 * 65) tab[q] = f * __ldg(&hg_eager_list.c[q]);
+    }
+    __syncwarp(kWarp30);
+  }
+};
+
+// Dynamic shared memory of a dop853_kernel<G> warp: in the looped form the
+// stage derivatives, then (G > 1) the step's products.
 template <int G>
 __host__ __device__ constexpr int dop_warp_doubles() {
-  return dop_looped<G>() ? 13 * Layout<G>::NC * 32 + (G > 1 ? dop_nnz() * Layout<G>::TPW : 0) : 0;
+  return G == 30 ? 3 * 13 * 5
+                 : (dop_looped<G>() ? 13 * Layout<G>::NC * 32 + (G > 1 ? dop_nnz() * Layout<G>::TPW : 0) : 0);
 }
 template <int G>
 __host__ __device__ constexpr size_t dop_smem_bytes(int block) {
@@ -1673,6 +1765,9 @@ __device__ __forceinline__ auto dop_coef(const Layout<G>& L, const double* tab, 
   } else if constexpr (dop_looped<G>()) {
     double* const t = sm_step + (threadIdx.x >> 5) * dop_warp_doubles<G>() + 13 * Layout<G>::NC * 32;
     return TableCoef<DopTab, G, Layout<G>::TPW>{t + (threadIdx.x & 31) / G, L.role, L.gmask};
+  } else if constexpr (G == 30) {
+    const int lane = threadIdx.x & 31;
+    return EagerCoef{sm_step + (threadIdx.x >> 5) * dop_warp_doubles<G>(), lane, lane / 6};
   } else if constexpr (G == 7) {
     return DopInlineCoef{0.0};  // no registers to spare for the shares
   } else {
@@ -1701,6 +1796,13 @@ __device__ __forceinline__ bool setup_layout(Layout<G>& L, Gather<G>& gat, doubl
     L.base = g * 6;
     L.gmask = 0x3Fu << L.base;
     traj = warp * 5 + g;
+  } else if constexpr (G == 30) {
+    if (lane >= 30) return false;
+    const int g = lane / 6;
+    L.role = lane % 6;
+    L.base = g * 6;
+    L.gmask = 0x3Fu << L.base;
+    traj = warp;
   } else if constexpr (G == 14) {
     if (lane >= 28) return false;
     const int g = lane / 14;
@@ -1730,6 +1832,7 @@ __host__ __device__ constexpr int gather_smem_doubles() {
 
 template <int G>
 __device__ __forceinline__ bool is_leader(const Layout<G>& L) {
+  if constexpr (G == 30) return L.role == 0 && L.base == 0;
   return (G == 1) || ((G == 2 || G == 6 || G == 14) && L.role == 0) || (G == 7 && L.role == 6);
 }
 
@@ -1813,7 +1916,10 @@ __device__ __forceinline__ void save_step(const Layout<G>& L, const DopParams& p
   constexpr int NC = Layout<G>::NC;
   int slot = 0;
   if (leader) slot = atomicAdd(p.refine_count, 1);
-  if constexpr (G > 1) slot = __shfl_sync(L.gmask, slot, leader_lane<G>(L));
+  if constexpr (G == 30)
+    slot = __shfl_sync(kWarp30, slot, 0);
+  else if constexpr (G > 1)
+    slot = __shfl_sync(L.gmask, slot, leader_lane<G>(L));
   double* r = p.rec + slot;
   const long long ld = p.rec_ld;
 #pragma unroll
@@ -1884,9 +1990,10 @@ __global__ void __launch_bounds__(128) dop853_kernel(DopParams p) {
   Gather<G> gat;
   int traj;
   __shared__ double sm_gather[gather_smem_doubles<G>()];  // 4 warps x 4 groups
-  __shared__ double sm_coef[dop_looped<G>() ? 1 : dop_nnz()];
+  constexpr bool shares = !dop_looped<G>() && G != 30;  // DopGroupCoef
+  __shared__ double sm_coef[shares ? dop_nnz() : 1];
   extern __shared__ double sm_step[];  // dop_smem_bytes<G>(blockDim.x)
-  if constexpr (!dop_looped<G>()) {
+  if constexpr (shares) {
     dop_coef_table_init(sm_coef);
     __syncthreads();
   }
@@ -1995,6 +2102,8 @@ __global__ void __launch_bounds__(128) dop853_kernel(DopParams p) {
       cf.set_step(h);
       if constexpr (dop_looped<G>())
         DopLane<G>::step_loop(L, y, cf, h, p.mu, p.dir, k, yh, e5, e3);
+      else if constexpr (G == 30)
+        DopLane<G>::step_eager(L, y, cf.tab + cf.g, h, p.mu, p.dir, k.v, yh, e5, e3);
       else
         DopLane<G>::step(L, y, cf, h, p.mu, p.dir, k.v, yh, e5, e3);
       double err_norm;
@@ -2029,13 +2138,31 @@ __global__ void __launch_bounds__(128) dop853_kernel(DopParams p) {
             const double hseg = t_new - t;
             double F[7][NC];
             DopLane<G>::dense_cache(L, y, yh, hseg, p.mu, p.dir, k, F);
-            while (q_next < p.m && (last || sample_t(q_next) < t_new)) {
-              const double x = (sample_t(q_next) - t) / hseg;
-              double* o = p.y_out + (long long)(p.dense_last ? 0 : q_next) * D * p.ld;
+            if constexpr (G == 30) {
+              // group g evaluates every fifth sample from q_next + g on; those
+              // of the step are a prefix of the rest
+              bool in = true;
+              while (in) {
+                const int q = q_next + cf.g;
+                in = q < p.m && (last || sample_t(q) < t_new);
+                if (in) {
+                  const double x = (sample_t(q) - t) / hseg;
+                  double* o = p.y_out + (long long)(p.dense_last ? 0 : q) * D * p.ld;
+                  o[(long long)L.comp(0) * p.ld + traj] = DopLane<G>::eval1(y[0], F, 0, x);
+                }
+                const int got = __popc(__ballot_sync(kWarp30, in)) / 6;
+                q_next += got;
+                in = got == 5;
+              }
+            } else {
+              while (q_next < p.m && (last || sample_t(q_next) < t_new)) {
+                const double x = (sample_t(q_next) - t) / hseg;
+                double* o = p.y_out + (long long)(p.dense_last ? 0 : q_next) * D * p.ld;
 #pragma unroll
-              for (int d = 0; d < NC; ++d)
-                o[(long long)L.comp(d) * p.ld + traj] = DopLane<G>::eval1(y[d], F, d, x);
-              ++q_next;
+                for (int d = 0; d < NC; ++d)
+                  o[(long long)L.comp(d) * p.ld + traj] = DopLane<G>::eval1(y[d], F, d, x);
+                ++q_next;
+              }
             }
           }
         }
@@ -2132,8 +2259,8 @@ __global__ void __launch_bounds__(128) dop853_kernel(DopParams p) {
     if constexpr (G == 1) {
       nt = atomicAdd(p.next_traj, 1) + p.stride;
     } else {
-      if (L.role == 0) nt = atomicAdd(p.next_traj, 1) + p.stride;
-      nt = __shfl_sync(L.gmask, nt, L.base);
+      if (G == 30 ? leader : L.role == 0) nt = atomicAdd(p.next_traj, 1) + p.stride;
+      nt = G == 30 ? __shfl_sync(kWarp30, nt, 0) : __shfl_sync(L.gmask, nt, L.base);
     }
     traj = nt;
   }

@@ -437,8 +437,10 @@ struct hg_server {
         const int g = lanes_for(d, live, sms);
         cudaError_t e;
         if (d == 6)
-          e = g == 6 ? segment<6>(p, live, sms, s)
-                     : (g == 2 ? segment<2>(p, live, sms, s) : segment<1>(p, live, sms, s));
+          e = g == 30  ? segment<30>(p, live, sms, s)
+              : g == 6 ? segment<6>(p, live, sms, s)
+              : g == 2 ? segment<2>(p, live, sms, s)
+                       : segment<1>(p, live, sms, s);
         else
           e = g == 14 ? segment<14>(p, live, sms, s) : segment<7>(p, live, sms, s);
         if (e == cudaSuccess && k.has_ev) e = d == 6 ? refine<1>(p, sms, s) : refine<7>(p, sms, s);
