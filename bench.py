@@ -76,7 +76,7 @@ def sched_lanes(n_live, warp_slots, sms=152):
     growing with the load beyond; among the layouts `lanes_d6` can fix, so 6
     where the driver gives a trajectory a whole warp)."""
     best, best_cost = 1, None
-    for g, per_warp, lat, cap in ((6, 5, 0.336, 5.15), (2, 16, 0.625, 5.05), (1, 32, 1.0, 4.35)):
+    for g, per_warp, lat, cap in ((6, 5, 0.337, 5.15), (2, 16, 0.634, 6.03), (1, 32, 1.0, 5.07)):
         load = -(-n_live // per_warp) / (cap * sms + 0.5 * (warp_slots - 3.0 * sms))
         cost = lat ** 4 * (1.0 + load ** 4)
         if best_cost is None or cost < best_cost:

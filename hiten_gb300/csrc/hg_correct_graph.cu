@@ -706,11 +706,10 @@ int lanes_d6(int n, int sms, int tuned) {
 }
 
 // STM leg layout: the handle's tuning, else the rule of event-free 42-dim runs
-// for two thirds of the orbits: they leave as they converge (2048 orbits: trio
-// 18.4 ms, pair 19.6; 4096: 30.5 and 26.3).
+// (2048 orbits: trio 17.0 ms, pair 19.1; 4096: 27.7 and 25.1).
 int lanes_d42(int tuned, int n, int sms) {
   if (tuned == 7 || tuned == 14 || tuned == 12 || tuned == 18) return tuned;
-  return hg_internal::lanes_d42_free(2LL * n / 3, sms, 3.0);
+  return hg_internal::lanes_d42_free(n, sms, 3.0);
 }
 
 void event_leg_any(int g, const Ws& w, double mu, const hg_newton_opts& o, int sms, cudaStream_t s, int* n) {

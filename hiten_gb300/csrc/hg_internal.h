@@ -29,15 +29,15 @@ int tuning(const hg_handle* h, int key);
 // both fits the measurements within 6 %) and grows with the warps per SM
 // beyond.  Measured on GB300 (us per DOP853 step, 152 SMs):
 //   n         1     608    912    1216   3040   4864   7296   9728   14592  19456  29184  48640
-//   1 lane    54.7  55.3   55.0   55.0   55.1   55.1   55.2   55.1   55.0   60.5   80.7   131
-//   2 lanes   31.1  34.4   34.5   34.5   34.4   34.5   34.5   37.3   45.1   57.0   83.5   138
-//   6 lanes   17.3  18.6   18.5   18.6   19.3   25.5   34.6   45.7   70.4   92.7   132    211
+//   1 lane    55.0  55.3   55.2   55.2   55.2   55.2   55.2   55.3   55.3   56.5   71.4   114
+//   2 lanes   31.8  35.0   35.0   35.0   35.0   35.1   35.2   35.8   41.6   50.0   97.5   140
+//   6 lanes   17.4  18.7   18.7   18.6   19.4   25.4   34.8   45.9   70.4   92.6   132    211
 //   30 lanes  15.1  16.1   17.4   21.2   (57 at 2280)
 // sm_capacity (the tuning value, 3 by default) moves the capacities.
 inline int lanes_d6(long long n, int sms, double sm_capacity) {
   const int gs[4] = {30, 6, 2, 1};
   const long long per_warp[4] = {1, 5, 16, 32};
-  const double lat[4] = {0.287, 0.336, 0.625, 1.0}, cap[4] = {6.6, 5.15, 5.05, 4.35};
+  const double lat[4] = {0.287, 0.337, 0.634, 1.0}, cap[4] = {6.6, 5.15, 6.03, 5.07};
   int best = 1;
   double best_cost = 0.0;
   for (int i = 0; i < 4; ++i) {
@@ -54,17 +54,17 @@ inline int lanes_d6(long long n, int sms, double sm_capacity) {
 }
 
 // Layout of an event-free single-pass 42-dim run of n trajectories: three warps
-// per five of them (18) while an SM holds at most two such groups, warp pairs
+// per five of them (18) while an SM holds at most three such groups, warp pairs
 // (12) beyond.  Measured on GB300 (us per step; G = 7 and 14 are behind at
 // every size):
-//   n              760    1000   1500   2048   4096   8192
-//   RK8, trio      28.5   35.2   35.2   50.3   100    178
-//   RK8, pair      40.5   40.9   41.0   45.8   82.9   165
-//   DOP853, trio   38.7   45.4   45.4   61.9   139    217
-//   DOP853, pair   52.2   52.8   52.9   58.2   98.6   195
+//   n              700    1000   1500   2048   4096   8192
+//   RK8, trio      28.9   32.6   32.6   42.4   77.4   142
+//   RK8, pair      40.4   40.6   40.6   43.3   74.2   155
+//   DOP853, trio   37.8   41.9   42.2   54.3   131    197
+//   DOP853, pair   52.0   52.6   52.7   56.2   91.1   180
 inline int lanes_d42_free(long long n, int sms, double sm_capacity) {
   const double groups = (double)((n + 4) / 5);
-  return groups <= 2.0 * (sm_capacity / 3.0) * sms ? 18 : 12;
+  return groups <= sm_capacity * sms ? 18 : 12;
 }
 
 }  // namespace hg_internal

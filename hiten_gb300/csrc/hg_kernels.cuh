@@ -93,37 +93,64 @@ __device__ __forceinline__ double neg_if(double v, bool neg) {
   return __longlong_as_double(__double_as_longlong(v) ^ (neg ? (long long)0x8000000000000000ull : 0ll));
 }
 
+// Products, sums and differences of a layout.  With four or more warps on an
+// SM its FP64 unit takes a multiply, an add, or a fused multiply-add with a
+// constant operand every 19.0 cycles, but a fused multiply-add of three
+// registers every 16.0 (measured, 4 to 32 warps); one warp alone waits 63.1 and
+// 64.6.  So the layouts that fill the unit form them as fused multiply-adds
+// with a neutral operand: a b + (-0), a 1 + b and (-b) 1 + a round once and have
+// the bits of a * b, a + b and a - b, signed zeros included.  The neutral
+// operands come by volatile loads: the compiler would fold known ones back.
+struct PlainOps {
+  __device__ __forceinline__ double mul(double a, double b) const { return a * b; }
+  __device__ __forceinline__ double add(double a, double b) const { return a + b; }
+  __device__ __forceinline__ double sub(double a, double b) const { return a - b; }
+};
+__device__ static double hg_neutral[2] = {1.0, -0.0};
+struct FusedOps {
+  double one, nz;
+  __device__ __forceinline__ FusedOps() {
+    asm volatile("ld.volatile.global.f64 %0, [%1];" : "=d"(one) : "l"(hg_neutral));
+    asm volatile("ld.volatile.global.f64 %0, [%1];" : "=d"(nz) : "l"(hg_neutral + 1));
+  }
+  __device__ __forceinline__ double mul(double a, double b) const { return fma(a, b, nz); }
+  __device__ __forceinline__ double add(double a, double b) const { return fma(a, one, b); }
+  __device__ __forceinline__ double sub(double a, double b) const { return fma(-b, one, a); }
+};
+
 // dynamics/rtbp.py:30-74 (_crtbp_accel), numba lowering of ** (x*x, x*(x*x)).
 // The distances and the six quotients over r1^3 and r2^3 are formed on the
 // FP32 and integer pipes (hg_exact.cuh): the bits of sqrt and `/`, with 31
 // FP64 instructions left of 75.
-__device__ __forceinline__ void rhs6(const double (&s)[6], double mu, double (&d)[6]) {
+__device__ __forceinline__ void rhs6(const FusedOps& o, const double (&s)[6], double mu, double (&d)[6]) {
   const double x = s[0], y = s[1], z = s[2], vx = s[3], vy = s[4];
   const double omu = 1.0 - mu;
   // What does not need the distances stands before the roots, so that its FP64
   // instructions run beside their integer sequences.
-  const double t1 = x + mu;
-  const double yy = y * y;
-  const double zz = z * z;
-  const double s1 = (t1 * t1 + yy) + zz;
-  const double t2 = x - omu;
-  const double s2 = (t2 * t2 + yy) + zz;
-  const double n1[3] = {omu * t1, omu * y, (-omu) * z};
-  const double n2[3] = {mu * ((x - 1.0) + mu), mu * y, mu * z};
-  const double cx = 2.0 * vy + x, cy = -2.0 * vx + y;
+  const double t1 = o.add(x, mu);
+  const double yy = o.mul(y, y);
+  const double zz = o.mul(z, z);
+  const double s1 = o.add(o.add(o.mul(t1, t1), yy), zz);
+  const double t2 = o.sub(x, omu);
+  const double s2 = o.add(o.add(o.mul(t2, t2), yy), zz);
+  const double n1[3] = {o.mul(omu, t1), o.mul(omu, y), o.mul(-omu, z)};
+  const double n2[3] = {o.mul(mu, o.add(o.sub(x, o.one), mu)), o.mul(mu, y), o.mul(mu, z)};
+  // 2 vy + x and -2 vx + y in one rounding each: the doubled velocity is exact
+  // (below the overflow of 2 v)
+  const double cx = fma(2.0, vy, x), cy = fma(-2.0, vx, y);
   const double r1 = hg_sqrt(s1);
   const double r2 = hg_sqrt(s2);
-  const double r1c = r1 * (r1 * r1);
-  const double r2c = r2 * (r2 * r2);
+  const double r1c = o.mul(r1, o.mul(r1, r1));
+  const double r2c = o.mul(r2, o.mul(r2, r2));
   double q1[3], q2[3];
   hg_quotients(n1, r1c, q1);
   hg_quotients(n2, r2c, q2);
   d[0] = vx;
   d[1] = vy;
   d[2] = s[5];
-  d[3] = (cx - q1[0]) - q2[0];
-  d[4] = (cy - q1[1]) - q2[1];
-  d[5] = q1[2] - q2[2];
+  d[3] = o.sub(o.sub(cx, q1[0]), q2[0]);
+  d[4] = o.sub(o.sub(cy, q1[1]), q2[1]);
+  d[5] = o.sub(q1[2], q2[2]);
 }
 
 // Hessian of the effective potential and the state accelerations,
@@ -178,6 +205,8 @@ struct Layout;
 
 template <>
 struct Layout<1> {
+  using Ops = FusedOps;
+  Ops ops;
   static constexpr int D = 6;
   static constexpr int NC = 6;    // components per lane
   static constexpr int TPW = 32;  // trajectories per warp
@@ -186,7 +215,7 @@ struct Layout<1> {
   int role;                       // always 6 ("state" lane of a 6-dim system)
   __device__ __forceinline__ int comp(int r) const { return r; }
   __device__ __forceinline__ void rhs(const double (&v)[6], double mu, const Dir& dir, double (&dv)[6]) const {
-    rhs6(v, mu, dv);
+    rhs6(ops, v, mu, dv);
 #pragma unroll
     for (int r = 0; r < 6; ++r)
       dv[r] = neg_if(dv[r], r >= dir.neg_lo && r < dir.neg_hi);
@@ -302,6 +331,8 @@ __device__ __forceinline__ Hess hessian_split(const LT& L, int job, double x, do
 
 template <>
 struct Layout<7> {
+  using Ops = PlainOps;
+  Ops ops;
   static constexpr int D = 42;
   static constexpr int NC = 6;
   static constexpr int TPW = 4;
@@ -327,8 +358,9 @@ struct Layout<7> {
       dv[0] = v[3];
       dv[1] = v[4];
       dv[2] = v[5];
-      dv[3] = ((H.xx * v[0] + H.xy * v[1]) + H.xz * v[2]) + 2.0 * v[4];
-      dv[4] = ((H.xy * v[0] + H.yy * v[1]) + H.yz * v[2]) + (-2.0) * v[3];
+      // (the doubled velocities are exact: one rounding)
+      dv[3] = fma(2.0, v[4], (H.xx * v[0] + H.xy * v[1]) + H.xz * v[2]);
+      dv[4] = fma(-2.0, v[3], (H.xy * v[0] + H.yy * v[1]) + H.yz * v[2]);
       dv[5] = (H.xz * v[0] + H.yz * v[1]) + H.zz * v[2];
     } else {
       dv[0] = v[3];
@@ -357,6 +389,8 @@ struct Layout<7> {
 // and operands as Layout<7>: same bits, at half the stage work per lane.
 template <>
 struct Layout<14> {
+  using Ops = PlainOps;
+  Ops ops;
   static constexpr int D = 42;
   static constexpr int NC = 3;
   static constexpr int TPW = 2;
@@ -376,12 +410,17 @@ struct Layout<14> {
     const Hess H = hessian_split(*this, role < 6 ? role : 0, x, y, z, vx, vy, mu);
     const int partner = role ^ 1;
     const double q0 = from(v[0], partner), q1 = from(v[1], partner), q2 = from(v[2], partner);
-    // rows 3..5 of F(x) Phi[:, c] (dynamics/rtbp.py:204-209): q = rows 0..2, v = rows 3..5
-    const double r3 = ((H.xx * q0 + H.xy * q1) + H.xz * q2) + 2.0 * v[1];
-    const double r4 = ((H.xy * q0 + H.yy * q1) + H.yz * q2) + (-2.0) * v[0];
-    const double r5 = (H.xz * q0 + H.yz * q1) + H.zz * q2;
+    // rows 3..5 of F(x) Phi[:, c] (dynamics/rtbp.py:204-209) from rows 0..2 (p)
+    // and the velocities: the odd lane forms row 3, the even lane row 4 in the
+    // same instructions and hands it over; both form row 5 (the doubled
+    // velocities are exact: one rounding)
     const bool pos = (role & 1) == 0, state = role >= 12;
-    double d0 = pos ? q0 : (state ? H.ax : r3);
+    const double p0 = pos ? v[0] : q0, p1 = pos ? v[1] : q1, p2 = pos ? v[2] : q2;
+    const double r34 = fma(pos ? -2.0 : 2.0, pos ? q0 : v[1],
+                           ((pos ? H.xy : H.xx) * p0 + (pos ? H.yy : H.xy) * p1) + (pos ? H.yz : H.xz) * p2);
+    const double r4 = from(r34, partner);
+    const double r5 = (H.xz * p0 + H.yz * p1) + H.zz * p2;
+    double d0 = pos ? q0 : (state ? H.ax : r34);
     double d1 = pos ? q1 : (state ? H.ay : r4);
     double d2 = pos ? q2 : (state ? H.az : r5);
     dv[0] = neg_if(d0, comp(0) >= dir.neg_lo && comp(0) < dir.neg_hi);
@@ -401,6 +440,8 @@ struct Layout<14> {
 // half that of G = 1, at ~7% more total work.
 template <>
 struct Layout<2> {
+  using Ops = FusedOps;
+  Ops ops;
   static constexpr int D = 6;
   static constexpr int NC = 3;
   static constexpr int TPW = 16;
@@ -423,19 +464,19 @@ struct Layout<2> {
     const double a2 = r0 ? 0.0 : mu;
     const double mb = r0 ? omu : mu;
     const double mz = r0 ? -omu : mu;
-    const double t = x + cb;
+    const double t = ops.add(x, cb);
     // y*y on role 0 and z*z on role 1 in one multiply, exchanged
     const double w = r0 ? y : z;
-    const double sq = w * w;
+    const double sq = ops.mul(w, w);
     const double sqo = __shfl_xor_sync(gmask, sq, 1);
     const double yy = r0 ? sq : sqo;
     const double zz = r0 ? sqo : sq;
     // what does not need the distance stands before its root (see rhs6)
-    const double s2 = (t * t + yy) + zz;
-    const double n[3] = {mb * ((x + a1) + a2), mb * y, mz * z};
+    const double s2 = ops.add(ops.add(ops.mul(t, t), yy), zz);
+    const double n[3] = {ops.mul(mb, ops.add(ops.add(x, a1), a2)), ops.mul(mb, y), ops.mul(mz, z)};
     const double r = hg_sqrt(s2);
-    const double rc = r * (r * r);
-    const double cor = (r0 ? 2.0 : -2.0) * (r0 ? vy : vx) + (r0 ? x : y);
+    const double rc = ops.mul(r, ops.mul(r, r));
+    const double cor = fma(r0 ? 2.0 : -2.0, r0 ? vy : vx, r0 ? x : y);
     double q[3];
     hg_quotients(n, rc, q);
     const double qx = q[0], qy = q[1], qz = q[2];
@@ -447,9 +488,9 @@ struct Layout<2> {
     const double pz = __shfl_xor_sync(gmask, qz, 1);
     const double q1 = r0 ? qx : p;
     const double q2 = r0 ? p : qy;
-    const double acc = (cor - q1) - q2;
+    const double acc = ops.sub(ops.sub(cor, q1), q2);
     const double ax = __shfl_xor_sync(gmask, acc, 1);
-    const double az = pz - qz;
+    const double az = ops.sub(pz, qz);
     dv[0] = r0 ? vx : ax;
     dv[1] = r0 ? vy : acc;
     dv[2] = r0 ? vz : az;
@@ -472,6 +513,8 @@ struct Layout<2> {
 // the per-step FP64 critical path is about 0.55x that of G = 2.
 template <>
 struct Layout<6> {
+  using Ops = PlainOps;
+  Ops ops;
   static constexpr int D = 6;
   static constexpr int NC = 1;
   static constexpr int TPW = 5;
@@ -864,19 +907,49 @@ __device__ __forceinline__ bool finite_bits(double a) {
 // instructions; one unrolled copy per stage makes a step larger than the
 // instruction cache, and a warp alone then runs at the rate of the fetches.
 // So the stages are a loop over the tableau's nonzero entries, listed by
-// rows: entry q is coefficient c[q] of derivative col[q]; row i (0 .. S - 1
+// rows: entry q is coefficient c[q] of the derivative in slot at[q]; row i (0 .. S - 1
 // the stages, S the weights) is [row[i], row[i + 1]).  Each sum has the terms
 // and the order of the unrolled form, so the bits too.
+// Derivatives share storage once they are done with: slot[j] is derivative
+// j's, free for another from the stage after its last use on (`keep`: used
+// beyond the stage sums); `slots` of them are needed (DOP853: 11 for 13, so that
+// twelve one-lane warps' fit an SM's shared memory).
 template <int S>
 struct StageList {
   static constexpr int kMax = (S + 1) * (S + 2) / 2;
   double c[kMax];
-  int col[kMax];
+  int at[kMax];  // slot of col
   int row[S + 2];
+  int slot[S + 1];
+  int slots;
 };
+// Derivatives a step's error norm, dense cache or next step reads (DOP853; none
+// for the fixed steps).
+template <class T>
+__host__ __device__ constexpr bool stage_keep(int j) {
+  if constexpr (std::is_same_v<T, DopTab>) {
+    bool used = j == 0 || j == 12 || T::e5(j) != 0.0 || T::e3(j) != 0.0;
+    for (int i = 13; i < 16; ++i) used = used || T::a(i, j) != 0.0;
+    for (int i = 0; i < 4; ++i) used = used || T::d(i, j) != 0.0;
+    return used;
+  }
+  return false;
+}
 template <class T>
 __host__ __device__ constexpr StageList<T::S> make_stage_list() {
   StageList<T::S> t{};
+  constexpr int N = std::is_same_v<T, DopTab> ? T::S + 1 : T::S;  // derivatives of a step
+  int busy_until[T::S + 1] = {};                                    // per slot: last stage that reads it
+  for (int j = 0; j < N; ++j) {
+    int last = stage_keep<T>(j) ? T::S + 2 : j;
+    for (int i = j + 1; i <= T::S; ++i)
+      if ((i < T::S ? T::a(i, j) : (j < T::S ? T::b(j) : 0.0)) != 0.0 && last < i) last = i;
+    int sl = 0;
+    while (sl < t.slots && busy_until[sl] > j) ++sl;  // written after stage j's sum
+    if (sl == t.slots) ++t.slots;
+    t.slot[j] = sl;
+    busy_until[sl] = last;
+  }
   int q = 0;
   for (int i = 0; i <= T::S; ++i) {
     t.row[i] = q;
@@ -884,12 +957,16 @@ __host__ __device__ constexpr StageList<T::S> make_stage_list() {
       const double v = i < T::S ? T::a(i, j) : T::b(j);
       if (v != 0.0) {
         t.c[q] = v;
-        t.col[q++] = j;
+        t.at[q++] = t.slot[j];
       }
     }
   }
   t.row[T::S + 1] = q;
   return t;
+}
+template <class T>
+__host__ __device__ constexpr int stage_slots() {
+  return make_stage_list<T>().slots;
 }
 template <class T>
 __host__ __device__ constexpr int stage_nnz() {
@@ -912,16 +989,22 @@ __device__ __forceinline__ const StageList<T::S>& stage_list() {
 }
 
 // The stage derivatives of a lane's components in shared memory,
-// lane-contiguous: derivative j, component d of a warp are 32 doubles.
+// lane-contiguous: component d of a slot is 32 doubles of a warp.
 template <int NC>
 struct StageRow {
   double* q;
   __device__ __forceinline__ double& operator[](int d) const { return q[d * 32]; }
 };
-template <int NC>
+template <class T, int NC>
 struct StageMem {
   double* p;
-  __device__ __forceinline__ StageRow<NC> operator[](int j) const { return StageRow<NC>{p + j * (NC * 32)}; }
+  __device__ __forceinline__ StageRow<NC> at(int slot) const { return StageRow<NC>{p + slot * (NC * 32)}; }
+  // derivative j, a compile-time constant
+  __device__ __forceinline__ StageRow<NC> operator[](int j) const {
+    constexpr StageList<T::S> tl = make_stage_list<T>();
+    return at(tl.slot[j]);
+  }
+  static constexpr int doubles = stage_slots<T>() * NC * 32;  // of a warp
 };
 
 // The products h c[q].  ListCoef: formed where they are used (one lane per
@@ -932,7 +1015,10 @@ template <class T>
 struct ListCoef {
   double h;
   __device__ __forceinline__ void set_step(double hh) { h = hh; }
-  __device__ __forceinline__ double product(int q) const { return h * stage_list<T>().c[q]; }
+  template <class Ops>
+  __device__ __forceinline__ double product(const Ops& ops, int q) const {
+    return ops.mul(h, stage_list<T>().c[q]);
+  }
 };
 template <class T, int NL, int STRIDE>
 struct TableCoef {
@@ -945,14 +1031,17 @@ struct TableCoef {
     for (int q = r; q < stage_nnz<T>(); q += NL) tab[q * STRIDE] = h * stage_list<T>().c[q];
     __syncwarp(gmask);
   }
-  __device__ __forceinline__ double product(int q) const { return tab[q * STRIDE]; }
+  template <class Ops>
+  __device__ __forceinline__ double product(const Ops&, int q) const {
+    return tab[q * STRIDE];
+  }
 };
 
 // y + sum of row i's products: the argument of stage i, or (i = S) the step's
 // end.  (Loading the next entry's operands under this one's sum was measured
 // too: 3 % slower for one and two lanes, level for six.)
-template <class T, int NC, class CF>
-__device__ __forceinline__ void stage_sum(int i, const double (&y)[NC], const CF& cf, const StageMem<NC>& k,
+template <class T, class Ops, int NC, class CF>
+__device__ __forceinline__ void stage_sum(const Ops& ops, int i, const double (&y)[NC], const CF& cf, const StageMem<T, NC>& k,
                                           double (&ys)[NC]) {
   const StageList<T::S>& tl = stage_list<T>();
 #pragma unroll
@@ -960,10 +1049,10 @@ __device__ __forceinline__ void stage_sum(int i, const double (&y)[NC], const CF
   const int end = tl.row[i + 1];
 #pragma unroll 1
   for (int q = tl.row[i]; q < end; ++q) {
-    const StageRow<NC> kr = k[tl.col[q]];
-    const double c = cf.product(q);
+    const StageRow<NC> kr = k.at(tl.at[q]);
+    const double c = cf.product(ops, q);
 #pragma unroll
-    for (int d = 0; d < NC; ++d) ys[d] = ys[d] + c * kr[d];
+    for (int d = 0; d < NC; ++d) ys[d] = ops.add(ys[d], ops.mul(c, kr[d]));
   }
 }
 
@@ -1022,19 +1111,20 @@ __device__ __forceinline__ void rk_fixed_step(const LT& L, const double (&y)[LT:
 // The same step with the stages as a loop.
 template <int ORDER, class LT, class CF>
 __device__ __forceinline__ void rk_fixed_step_loop(const LT& L, const double (&y)[LT::NC], const CF& cf, double mu,
-                                                   const Dir& dir, const StageMem<LT::NC>& k, double (&yn)[LT::NC]) {
+                                                   const Dir& dir, const StageMem<FixedTab<ORDER>, LT::NC>& k,
+                                                   double (&yn)[LT::NC]) {
   using T = FixedTab<ORDER>;
   constexpr int NC = LT::NC;
 #pragma unroll 1
   for (int i = 0; i < T::S; ++i) {
     double ys[NC], kt[NC];
-    stage_sum<T>(i, y, cf, k, ys);
+    stage_sum<T>(L.ops, i, y, cf, k, ys);
     L.rhs(ys, mu, dir, kt);
-    const StageRow<NC> kr = k[i];
+    const StageRow<NC> kr = k.at(stage_list<T>().slot[i]);
 #pragma unroll
     for (int d = 0; d < NC; ++d) kr[d] = kt[d];
   }
-  stage_sum<T>(T::S, y, cf, k, yn);
+  stage_sum<T>(L.ops, T::S, y, cf, k, yn);
 }
 
 template <int ORDER, class LT>
@@ -1188,7 +1278,7 @@ __global__ void __launch_bounds__(128) fixed_rk_event_kernel(FixedParams p) {
 // 13.7 -> 7.5, 40000 34.1 -> 19.7; RK8 61.3 -> 18.2, 61.3 -> 34.0, 161 -> 109.
 template <int ORDER, int G>
 __host__ __device__ constexpr int fixed_warp_doubles() {
-  return FixedTab<ORDER>::S * Layout<G>::NC * 32 + stage_nnz<FixedTab<ORDER>>();
+  return StageMem<FixedTab<ORDER>, Layout<G>::NC>::doubles + stage_nnz<FixedTab<ORDER>>();
 }
 template <int ORDER, int G>
 __host__ __device__ constexpr size_t fixed_smem_bytes(int block) {
@@ -1214,8 +1304,8 @@ __global__ void __launch_bounds__(128) fixed_rk_d6_kernel(FixedParams p) {
   const int traj = warp * TPW + g < p.N ? warp * TPW + g : p.N - 1;
   const bool writes = lane < TPW * G && warp * TPW + g < p.N;
   double* const sm = sm_step + (threadIdx.x >> 5) * fixed_warp_doubles<ORDER, G>();
-  const StageMem<NC> k{sm + lane};
-  TableCoef<T, 32, 1> cf{sm + T::S * NC * 32, lane, 0xFFFFFFFFu};
+  const StageMem<T, NC> k{sm + lane};
+  TableCoef<T, 32, 1> cf{sm + StageMem<T, NC>::doubles, lane, 0xFFFFFFFFu};
   double y[NC];
 #pragma unroll
   for (int r = 0; r < NC; ++r) y[r] = p.y0[(long long)L.comp(r) * p.ld_in + traj];
@@ -1523,7 +1613,7 @@ struct DopLaneT {
   static constexpr int NC = LT::NC;
   // err5 / err3 of a step, from k[0..12]
   template <class K>
-  __device__ __forceinline__ static void error_sums(const K& k, double h, double (&e5)[NC], double (&e3)[NC]) {
+  __device__ __forceinline__ static void error_sums(const LT& L, const K& k, double h, double (&e5)[NC], double (&e3)[NC]) {
     using T = DopTab;
     // err5 = sum_j E5_j k_j (the reference starts from zeros; the first term
     // is taken as the start here: only the sign of an all-zero sum can
@@ -1535,12 +1625,12 @@ struct DopLaneT {
       if constexpr (c5 != 0.0) {
         constexpr bool first = dop_first_nonzero_e(true) == j;
 #pragma unroll
-        for (int d = 0; d < NC; ++d) e5[d] = first ? c5 * k[j][d] : e5[d] + c5 * k[j][d];
+        for (int d = 0; d < NC; ++d) e5[d] = first ? c5 * k[j][d] : L.ops.add(e5[d], L.ops.mul(c5, k[j][d]));
       }
       if constexpr (c3 != 0.0) {
         constexpr bool first = dop_first_nonzero_e(false) == j;
 #pragma unroll
-        for (int d = 0; d < NC; ++d) e3[d] = first ? c3 * k[j][d] : e3[d] + c3 * k[j][d];
+        for (int d = 0; d < NC; ++d) e3[d] = first ? c3 * k[j][d] : L.ops.add(e3[d], L.ops.mul(c3, k[j][d]));
       }
     });
 #pragma unroll
@@ -1586,18 +1676,18 @@ struct DopLaneT {
   // exit.
   template <class CF>
   __device__ __forceinline__ static void step_loop(const LT& L, const double (&y)[NC], const CF& cf, double h,
-                                                   double mu, const Dir& dir, const StageMem<NC>& k,
+                                                   double mu, const Dir& dir, const StageMem<DopTab, NC>& k,
                                                    double (&yh)[NC], double (&e5)[NC], double (&e3)[NC]) {
 #pragma unroll 1
     for (int i = 1; i <= DopTab::S; ++i) {
-      stage_sum<DopTab>(i, y, cf, k, yh);
+      stage_sum<DopTab>(L.ops, i, y, cf, k, yh);
       double kt[NC];
       L.rhs(yh, mu, dir, kt);
-      const StageRow<NC> kr = k[i];
+      const StageRow<NC> kr = k.at(stage_list<DopTab>().slot[i]);
 #pragma unroll
       for (int d = 0; d < NC; ++d) kr[d] = kt[d];
     }
-    error_sums(k, h, e5, e3);
+    error_sums(L, k, h, e5, e3);
   }
   // one attempted DOP853 step; k[0] = f(t, y) on entry; k[12] = f(t+h, y_high)
   // on exit; the products h * a_ij, h * b_j from `cf` (set for h)
@@ -1632,7 +1722,7 @@ struct DopLaneT {
       }
     });
     L.rhs(yh, mu, dir, k[12]);
-    error_sums(k, h, e5, e3);
+    error_sums(L, k, h, e5, e3);
   }
 
   // _dop853_build_dense_cache: F[0..6][6] for this lane's components.
@@ -1751,7 +1841,8 @@ struct EagerCoef {
 template <int G>
 __host__ __device__ constexpr int dop_warp_doubles() {
   return G == 30 ? 3 * 13 * 5
-                 : (dop_looped<G>() ? 13 * Layout<G>::NC * 32 + (G > 1 ? dop_nnz() * Layout<G>::TPW : 0) : 0);
+                 : (dop_looped<G>() ? StageMem<DopTab, Layout<G>::NC>::doubles + (G > 1 ? dop_nnz() * Layout<G>::TPW : 0)
+                                    : 0);
 }
 template <int G>
 __host__ __device__ constexpr size_t dop_smem_bytes(int block) {
@@ -1763,7 +1854,8 @@ __device__ __forceinline__ auto dop_coef(const Layout<G>& L, const double* tab, 
   if constexpr (G == 1) {
     return ListCoef<DopTab>{0.0};
   } else if constexpr (dop_looped<G>()) {
-    double* const t = sm_step + (threadIdx.x >> 5) * dop_warp_doubles<G>() + 13 * Layout<G>::NC * 32;
+    double* const t =
+        sm_step + (threadIdx.x >> 5) * dop_warp_doubles<G>() + StageMem<DopTab, Layout<G>::NC>::doubles;
     return TableCoef<DopTab, G, Layout<G>::TPW>{t + (threadIdx.x & 31) / G, L.role, L.gmask};
   } else if constexpr (G == 30) {
     const int lane = threadIdx.x & 31;
@@ -1927,8 +2019,11 @@ __device__ __forceinline__ void save_step(const Layout<G>& L, const DopParams& p
     const int c = L.comp(d);
     r[c * ld] = y[d];
     r[(D + c) * ld] = yh[d];
-#pragma unroll
-    for (int j = 0; j < 13; ++j) r[(2 * D + j * D + c) * ld] = k[j][d];
+    // k_1 .. k_4 enter nothing after the stages
+    static_for<13>([&](auto jc) {
+      constexpr int j = decltype(jc)::value;
+      if constexpr (stage_keep<DopTab>(j)) r[(2 * D + j * D + c) * ld] = k[j][d];
+    });
   }
   if (leader) {
     r[(15 * D) * ld] = h;
@@ -1964,8 +2059,10 @@ __global__ void __launch_bounds__(128) refine_kernel(DopParams p) {
       const int c = L.comp(d);
       y[d] = r[c * ld];
       yh[d] = r[(D + c) * ld];
-#pragma unroll
-      for (int j = 0; j < 13; ++j) k[j][d] = r[(2 * D + j * D + c) * ld];
+      static_for<13>([&](auto jc) {
+        constexpr int j = decltype(jc)::value;
+        k[j][d] = stage_keep<DopTab>(j) ? r[(2 * D + j * D + c) * ld] : 0.0;
+      });
     }
     const double h = r[(15 * D) * ld];
     const double t = r[(15 * D + 1) * ld];
@@ -1981,9 +2078,12 @@ __global__ void __launch_bounds__(128) refine_kernel(DopParams p) {
 }
 
 // DENSE = false compiles the dense-output path out (launches without
-// samples): fewer live registers in the step loop.
+// samples): fewer live registers in the step loop.  One lane per trajectory:
+// twelve warps per SM, three on each sub-partition (168 registers; what spills
+// are the error sums, once per step) -- ten warps, two or three on each, took
+// the FP64 unit unevenly.
 template <int G, bool DENSE = true>
-__global__ void __launch_bounds__(128) dop853_kernel(DopParams p) {
+__global__ void __launch_bounds__(128, G == 1 && !DENSE ? 3 : 1) dop853_kernel(DopParams p) {
   constexpr int D = Layout<G>::D;
   constexpr int NC = Layout<G>::NC;
   Layout<G> L;
@@ -2001,7 +2101,7 @@ __global__ void __launch_bounds__(128) dop853_kernel(DopParams p) {
   const bool leader = is_leader<G>(L);
   const bool has_event = p.ev_index >= 0 && p.max_hits > 0;
   const EvCtx<G> ev(L, has_event ? p.ev_index : -1);
-  std::conditional_t<dop_looped<G>(), StageMem<NC>, StageRegs<NC>> k;
+  std::conditional_t<dop_looped<G>(), StageMem<DopTab, NC>, StageRegs<NC>> k;
   auto cf = dop_coef<G>(L, sm_coef, sm_step);
   if constexpr (dop_looped<G>()) k.p = sm_step + (threadIdx.x >> 5) * dop_warp_doubles<G>() + (threadIdx.x & 31);
 

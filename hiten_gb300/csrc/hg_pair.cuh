@@ -135,6 +135,8 @@ struct PairLane {
 
 // State warp: one state component per lane (NC = 1).
 struct PairState {
+  using Ops = PlainOps;
+  Ops ops;
   static constexpr int D = 42;
   static constexpr int NC = 1;
   static constexpr bool kState = true;
@@ -174,6 +176,8 @@ struct PairState {
 
 // STM warp: one column of Phi per lane (NC = 6, rows 0..5).
 struct PairStm {
+  using Ops = FusedOps;
+  Ops ops;
   static constexpr int D = 42;
   static constexpr int NC = 6;
   static constexpr bool kState = false;
@@ -208,9 +212,11 @@ struct PairStm {
     dv[0] = v[3];
     dv[1] = v[4];
     dv[2] = v[5];
-    dv[3] = ((xx * v[0] + xy * v[1]) + xz * v[2]) + 2.0 * v[4];
-    dv[4] = ((xy * v[0] + yy * v[1]) + yz * v[2]) + (-2.0) * v[3];
-    dv[5] = (xz * v[0] + yz * v[1]) + zz * v[2];
+    // (the doubled velocities are exact: one rounding)
+    const Ops& o = ops;
+    dv[3] = fma(2.0, v[4], o.add(o.add(o.mul(xx, v[0]), o.mul(xy, v[1])), o.mul(xz, v[2])));
+    dv[4] = fma(-2.0, v[3], o.add(o.add(o.mul(xy, v[0]), o.mul(yy, v[1])), o.mul(yz, v[2])));
+    dv[5] = o.add(o.add(o.mul(xz, v[0]), o.mul(yz, v[1])), o.mul(zz, v[2]));
 #pragma unroll
     for (int r = 0; r < 6; ++r) {
       const int c = comp(r);
@@ -228,6 +234,8 @@ struct PairStm {
 // six-lane group for the step control (coefficients, norms, step-size
 // factor), so each trajectory's two halves take the same decisions.
 struct PairStmHalf {
+  using Ops = FusedOps;
+  Ops ops;
   static constexpr int D = 42;
   static constexpr int NC = 3;
   static constexpr bool kState = false;
@@ -264,12 +272,18 @@ struct PairStmHalf {
     // the partner lane (lane ^ 1) holds the other rows of the column
     const double q0 = __shfl_xor_sync(gmask, v[0], 1), q1 = __shfl_xor_sync(gmask, v[1], 1),
                  q2 = __shfl_xor_sync(gmask, v[2], 1);
-    // rows 3..5 of F(x) Phi[:, c] (dynamics/rtbp.py:204-209), as Layout<14>
-    const double r3 = ((xx * q0 + xy * q1) + xz * q2) + 2.0 * v[1];
-    const double r4 = ((xy * q0 + yy * q1) + yz * q2) + (-2.0) * v[0];
-    const double r5 = (xz * q0 + yz * q1) + zz * q2;
+    // rows 3..5 of F(x) Phi[:, c] (dynamics/rtbp.py:204-209), as Layout<14>:
+    // the odd lane forms row 3, the even lane row 4 in the same instructions
+    // and hands it over; both form row 5
     const bool pos = ((role % 6) & 1) == 0;
-    const double d0 = pos ? q0 : r3, d1 = pos ? q1 : r4, d2 = pos ? q2 : r5;
+    const double p0 = pos ? v[0] : q0, p1 = pos ? v[1] : q1, p2 = pos ? v[2] : q2;
+    const double w = pos ? q0 : v[1];  // row 3 takes 2 v4, row 4 -2 v3
+    const Ops& o = ops;
+    const double r34 = fma(pos ? -2.0 : 2.0, w, o.add(o.add(o.mul(pos ? xy : xx, p0), o.mul(pos ? yy : xy, p1)),
+                                                      o.mul(pos ? yz : xz, p2)));
+    const double r4 = __shfl_xor_sync(gmask, r34, 1);
+    const double r5 = o.add(o.add(o.mul(xz, p0), o.mul(yz, p1)), o.mul(zz, p2));
+    const double d0 = pos ? q0 : r34, d1 = pos ? q1 : r4, d2 = pos ? q2 : r5;
     dv[0] = neg_if(d0, comp(0) >= dir.neg_lo && comp(0) < dir.neg_hi);
     dv[1] = neg_if(d1, comp(1) >= dir.neg_lo && comp(1) < dir.neg_hi);
     dv[2] = neg_if(d2, comp(2) >= dir.neg_lo && comp(2) < dir.neg_hi);
@@ -283,7 +297,7 @@ struct PairStmHalf {
 // derivatives, the step's products).
 template <int ORDER>
 __host__ __device__ constexpr int pair_fixed_doubles(int nc) {
-  return FixedTab<ORDER>::S * nc * 32 + stage_nnz<FixedTab<ORDER>>();
+  return stage_slots<FixedTab<ORDER>>() * nc * 32 + stage_nnz<FixedTab<ORDER>>();
 }
 template <int ORDER, class LT>
 __device__ __forceinline__ bool pair_fixed_run(const LT& L, const FixedParams& p, int traj, bool writes, double* sm) {
@@ -297,8 +311,9 @@ __device__ __forceinline__ bool pair_fixed_run(const LT& L, const FixedParams& p
   }
   const long long row = 42LL * p.ld_out;
   bool finite = true;
-  const StageMem<NC> k{sm + (threadIdx.x & 31)};
-  TableCoef<FixedTab<ORDER>, 32, 1> cf{sm + FixedTab<ORDER>::S * NC * 32, (int)(threadIdx.x & 31), 0xFFFFFFFFu};
+  using T = FixedTab<ORDER>;
+  const StageMem<T, NC> k{sm + (threadIdx.x & 31)};
+  TableCoef<T, 32, 1> cf{sm + StageMem<T, NC>::doubles, (int)(threadIdx.x & 31), 0xFFFFFFFFu};
   for (int idx = 0; idx < p.n - 1; ++idx) {
     const double h = p.t_vals[idx + 1] - p.t_vals[idx];
     cf.set_step(h);
@@ -511,7 +526,9 @@ __device__ __forceinline__ void pair_exchange(const LT& L, PairGather* gx, unsig
 }
 
 // Shared memory of a warp: stage derivatives, then its groups' products.
-__host__ __device__ constexpr int pair_dop_doubles(int nc) { return 13 * nc * 32 + stage_nnz<DopTab>() * kPairTraj; }
+__host__ __device__ constexpr int pair_dop_doubles(int nc) {
+  return stage_slots<DopTab>() * nc * 32 + stage_nnz<DopTab>() * kPairTraj;
+}
 // A pair's link, gather slots and both warps' parts.
 __host__ __device__ constexpr size_t pair_dop_bytes() {
   return sizeof(PairLink) + sizeof(PairGather) + (pair_dop_doubles(1) + pair_dop_doubles(6)) * sizeof(double);
@@ -542,7 +559,7 @@ __device__ __forceinline__ bool pair_dop_run(const LT& L, const DopParams& p, Pa
   double y[NC];
 #pragma unroll
   for (int r = 0; r < NC; ++r) y[r] = p.y0[(long long)L.comp(r) * p.ld + traj];
-  const StageMem<NC> k{sm + (threadIdx.x & 31)};
+  const StageMem<DopTab, NC> k{sm + (threadIdx.x & 31)};
   double k0[NC];
   L.rhs(y, p.mu, p.dir, k0);
 #pragma unroll
@@ -574,7 +591,7 @@ __device__ __forceinline__ bool pair_dop_run(const LT& L, const DopParams& p, Pa
   // integrators/rk.py loop test (t - t_end) * direction < 0, direction +1
   bool live = running && hg_lt0(t - tmax);
   // (the shadow lanes of group 4 write their role's entries again)
-  TableCoef<DopTab, 6, kPairTraj> cf{sm + 13 * NC * 32 + L.base / 6, L.role % 6, L.gmask};
+  TableCoef<DopTab, 6, kPairTraj> cf{sm + StageMem<DopTab, NC>::doubles + L.base / 6, L.role % 6, L.gmask};
   while (vote_any(live)) {
     bool go = live;
     if (go && (long long)(acc + rej) >= p.max_steps) {
