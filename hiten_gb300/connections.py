@@ -65,9 +65,9 @@ class GpuSectionMatcher:
         nq, nr = q.shape[0], r.shape[0]
         qx, qy = self._xy(q)
         rx, ry = self._xy(r)
-        cnt = torch.empty(nq, dtype=torch.int32, device=self.device)
-        bi = torch.empty(nq, dtype=torch.int32, device=self.device)
-        bd = torch.empty(nq, dtype=torch.float64, device=self.device)
+        # one buffer, read back in one copy
+        out = torch.empty(16 * nq, dtype=torch.uint8, device=self.device)
+        bd, cnt, bi = out[:8 * nq], out[8 * nq:12 * nq], out[12 * nq:]
         st = C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
         ws, wsb = self._workspace(L, nr)
         with torch.cuda.device(self.device):
@@ -75,7 +75,9 @@ class GpuSectionMatcher:
                                   P._ptr(cnt), P._ptr(bi), P._ptr(bd), P._ptr(ws), wsb, st)
         if rc != _lib.HG_OK:
             raise _lib.HitenGpuError(rc, "hg_radius_best failed")
-        return cnt.cpu().numpy().astype(np.int64), bi.cpu().numpy().astype(np.int64), bd.cpu().numpy()
+        host = out.cpu().numpy()
+        return (host[8 * nq:12 * nq].view(np.int32).astype(np.int64), host[12 * nq:].view(np.int32).astype(np.int64),
+                host[:8 * nq].view(np.float64))
 
     def nearest(self, p, coord_max):
         L = _lib.load()
