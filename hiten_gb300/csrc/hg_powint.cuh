@@ -116,14 +116,34 @@ HG_XHD double hgp_exp(const HgLog2& g, uint64_t Y, bool neg, bool& ok) {
 //     3.4 units (x^1.5), 2 (1.2 + 1 + 0.5) = 5.4 (x^2.5).
 // Closer than that to a rounding boundary (one value in 256 and in 170) `ok`
 // is cleared.
-HG_XHD double hgp_pow15_or_25(double x, float y, bool want25, bool& ok) {
+// sqrt(x)'s significand s in 64 bits.
+HG_XHD uint64_t hgp_root64(double x, float y) {
   uint64_t S_raw;
   float fr;
   hgx_sqrt_parts(x, y, S_raw, fr);
+  return ((S_raw - ((uint64_t)HGX_OFFSET << 32)) << 11) +
+         (uint64_t)(int64_t)(int32_t)(hgx_fbits(fmaf(fr, 2048.0f, HGX_M2)) - HGX_M2_BITS);
+}
+// x's significand in 64 bits
+HG_XHD uint64_t hgp_significand64(double x) {
   const uint32_t hi = hgx_hi(x), lo = hgx_lo(x);
-  const uint64_t S = ((S_raw - ((uint64_t)HGX_OFFSET << 32)) << 11) +
-                     (uint64_t)(int64_t)(int32_t)(hgx_fbits(fmaf(fr, 2048.0f, HGX_M2)) - HGX_M2_BITS);
-  const uint64_t m = ((uint64_t)(((hi & 0xFFFFFu) | 0x100000u) << 11 | lo >> 21) << 32) | (lo << 11);
+  return ((uint64_t)(((hi & 0xFFFFFu) | 0x100000u) << 11 | lo >> 21) << 32) | (lo << 11);
+}
+// The power from its significand R (upper 53 bits, rounded) and exponent: e +
+// floor(e / 2), or 2 e + floor(e / 2), plus one for every product that reached
+// 2 (sm, sr: those that did not).
+HG_XHD double hgp_make_power(double x, uint64_t R, bool want25, uint32_t sm, uint32_t sr) {
+  const int32_t e = (int32_t)(hgx_hi(x) >> 20) - 1023;
+  const int32_t ex = e + (e >> 1) + (want25 ? e + 1 - (int32_t)sm : 0) + 1 - (int32_t)sr;
+  const uint64_t q = ((R >> 10) + 1u) >> 1;
+  const uint64_t bits = q + ((uint64_t)(uint32_t)(ex + 1022) << 52);
+  return hgx_make((uint32_t)(bits >> 32), (uint32_t)bits);
+}
+// |e| < 100: the powers stay far from the ends of the range
+HG_XHD bool hgp_power_range(double x) { return (hgx_hi(x) - (923u << 20)) < (200u << 20); }
+
+HG_XHD double hgp_pow15_or_25(double x, float y, bool want25, bool& ok) {
+  const uint64_t S = hgp_root64(x, y), m = hgp_significand64(x);
   uint64_t mm = hgp_mulhi64(m, m);
   const uint32_t sm = (uint32_t)(~mm >> 63);  // m^2 < 2
   mm = (mm << sm) + sm;
@@ -131,24 +151,58 @@ HG_XHD double hgp_pow15_or_25(double x, float y, bool want25, bool& ok) {
   uint64_t R = hgp_mulhi64(W, S);
   const uint32_t sr = (uint32_t)(~R >> 63);
   R = (R << sr) + sr;
-  // exponent: e + floor(e / 2), or 2 e + floor(e / 2), plus one for every
-  // product that reached 2
-  const int32_t e = (int32_t)(hi >> 20) - 1023;
-  const int32_t ex = e + (e >> 1) + (want25 ? e + 1 - (int32_t)sm : 0) + 1 - (int32_t)sr;
-  const uint64_t q = ((R >> 10) + 1u) >> 1;
   const uint32_t w = want25 ? 6u : 4u;
-  // |e| < 100: the powers stay far from the ends of the range
-  ok = (hi - (923u << 20)) < (200u << 20) && (((uint32_t)R + 1024u + w) & 2047u) >= 2u * w;
-  const uint64_t bits = q + ((uint64_t)(uint32_t)(ex + 1022) << 52);
-  return hgx_make((uint32_t)(bits >> 32), (uint32_t)bits);
+  ok = hgp_power_range(x) && (((uint32_t)R + 1024u + w) & 2047u) >= 2u * w;
+  return hgp_make_power(x, R, want25, sm, sr);
+}
+
+// The same power for an `x` whose `ok` was cleared, with 30 more bits of the
+// root: r = s^2 - S^2, exact modulo 2^128 and below 2^66, gives the root's
+// next correction r / (2 S), an integer d in units of 2^-93, off by at most
+// 1.2 * 2^30 * 2^-22.2 (y and two FP32 roundings) + 2 + 0.5 < 320.  The product
+// with m (exact) or m^2 (106 bits, exact) in 128 bits is then off by less than
+// 2 (320 * 2^34 + 3) = 2^43.4 units of its last bit, 2^-20.6 of R's.  `ok`
+// stays cleared only within 2^-20 of a boundary.  A warp of five 42-dim
+// trajectories takes twenty powers a right-hand side, so one right-hand side in
+// ten came to the double-double form's forty FP64 instructions; with this form
+// in between: fixed RK8 of 1024 states, 3000 steps, 98.7 -> 97.0 ms; 97
+// monodromy matrices 2.76 -> 2.72 ms.
+HG_XHD double hgp_pow15_or_25_wide(double x, float y, bool want25, bool& ok) {
+  typedef unsigned __int128 u128;
+  const uint64_t S = hgp_root64(x, y), m = hgp_significand64(x);
+  const uint32_t odd = ~(hgx_hi(x) >> 20) & 1u;  // s^2 is m, or 2 m for an odd exponent
+  const u128 r = ((u128)m << (63u + odd)) - (u128)S * S;
+  const float rf = (float)(int32_t)(uint32_t)(uint64_t)(r >> 35);
+  const int64_t d = (int64_t)rintf(rf * (2.0f * y));
+  const u128 root = ((u128)S << 64) + (u128)((__int128)d << 34);
+  const uint64_t Sh = (uint64_t)(root >> 64), Sl = (uint64_t)root;
+  u128 W = (u128)m << 64;
+  uint32_t sm = 0u;
+  if (want25) {
+    W = (u128)m * m;
+    sm = (uint32_t)(~(uint64_t)(W >> 64) >> 63);
+    W <<= sm;
+  }
+  const uint64_t Wh = (uint64_t)(W >> 64), Wl = (uint64_t)W;
+  u128 P = (u128)Wh * Sh + hgp_mulhi64(Wl, Sh) + hgp_mulhi64(Wh, Sl);
+  const uint32_t sr = (uint32_t)(~(uint64_t)(P >> 64) >> 63);
+  P <<= sr;
+  const uint64_t R = (uint64_t)(P >> 64);
+  const uint64_t low = ((R & 2047u) << 32) | (uint32_t)((uint64_t)P >> 32);  // in units of 2^-32 of R's
+  ok = hgp_power_range(x) && low - (1024ull << 32) + 4096u >= 8192u;
+  return hgp_make_power(x, R, want25, sm, sr);
 }
 
 #if defined(__CUDACC__)
-// x^1.5 or x^2.5, with the double-double form behind it
+// x^1.5 or x^2.5, with the wider root and the double-double form behind it
 __device__ __forceinline__ double hg_power_of_r2(double x, bool want25) {
   bool ok;
-  double p = hgp_pow15_or_25(x, hgx_rsqrt_approx(hgx_sqrt_arg(x)), want25, ok);
-  if (!ok) p = hg_pow15_or_25(x, want25);
+  const float y = hgx_rsqrt_approx(hgx_sqrt_arg(x));
+  double p = hgp_pow15_or_25(x, y, want25, ok);
+  if (!ok) {
+    p = hgp_pow15_or_25_wide(x, y, want25, ok);
+    if (!ok) p = hg_pow15_or_25(x, want25);
+  }
   return p;
 }
 #endif
