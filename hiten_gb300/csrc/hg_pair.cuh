@@ -149,11 +149,13 @@ struct PairState {
   __device__ __forceinline__ int comp(int) const { return 36 + (role < 6 ? role : 0); }
   __device__ __forceinline__ double from(double v, int r) const { return __shfl_sync(gmask, v, base + r); }
   __device__ __forceinline__ void rhs(const double (&v)[1], double mu, const Dir& dir, double (&dv)[1]) const {
+    const int job = role < 6 ? role : 0;  // (the shadow lanes repeat job 0 in full)
     const double x = from(v[0], 0), y = from(v[0], 1), z = from(v[0], 2);
-    const double vx = from(v[0], 3), vy = from(v[0], 4);
-    // position lanes: their derivative is the velocity of lane role + 3
-    const double u = from(v[0], role < 3 ? role + 3 : 0);
-    const Hess H = hessian_split<PairState, false>(*this, role < 6 ? role : 0, x, y, z, vx, vy, mu);
+    // position lanes: their derivative is the velocity of lane job + 3; lane 3
+    // takes vy, lane 4 vx
+    const double u = from(v[0], nibble(0x534543u, job));
+    double off;
+    const double form = hessian_job(job, x, y, z, u, mu, off);
     const unsigned b = seq % kPairSlots, use = seq / kPairSlots;
     if (!broken && use >= 1) {
       // the slot's previous contents must have been read (a warp-uniform outcome)
@@ -161,16 +163,81 @@ struct PairState {
       broken = !__all_sync(0xFFFFFFFFu, ok);
     }
     if (!broken) {
-      // the six Hessian entries xx, yy, zz, xy, yz, xz: lanes 3..5 formed
-      // the off-diagonal ones as hessian42 does (H.xy holds this lane's)
-      const double off = H.xy;
-      if (role < 6) link->H[b][t][role] = role == 0 ? H.xx : (role == 1 ? H.yy : (role == 2 ? H.zz : off));
+      // the six Hessian entries xx, yy, zz, xy, yz, xz
+      if (role < 6) link->H[b][t][role] = role < 3 ? form : off;
       mbar_arrive(&link->full[b]);
     }
     ++seq;
-    const double d = role < 3 ? u : (role == 3 ? H.ax : (role == 4 ? H.ay : H.az));
+    const double d = job < 3 ? u : form;
     const int c = comp(0);
     dv[0] = neg_if(d, c >= dir.neg_lo && c < dir.neg_hi);
+  }
+  static __device__ __forceinline__ int nibble(unsigned table, int job) { return (int)(table >> (4 * job)) & 7; }
+  // hessian_split's work with each lane keeping its own entry: returns xx, yy,
+  // zz, ax, ay, az for jobs 0..5 and sets `off` to xy, yz, xz on jobs 3..5.
+  // Lane 3 b + k (b = primary, k < 3) takes the power of its primary its two
+  // quotients divide by:
+  //   0: mu2/r3, t1/r3     1: y/r3, z/r3     2: mu2/r5, (mu2 t1)/r5
+  //   3: mu/R3,  t2/R3     4: y/R3, z/R3     5: mu/R5,  (mu t2)/R5
+  // A job needs four of the twelve, two for a sum (s1 + s2) and two as factors
+  // (f1, f2); four shuffles hand them out, each lane offering in each the one
+  // its readers want.  The expressions and operands are hessian42's (x - m == x +
+  // (-m), (-a) u == -(a u), -0 + v == v, a + b == b + a): same bits.  `u`: vy
+  // on job 3, vx on job 4.  The state warp's chain is what a step of the trio
+  // waits for (its STM warps alone would take 23.3 us of an RK8 step's 28.9):
+  // twelve shuffles here and in rhs instead of the 26 of hessian_split and its
+  // caller, and their selects, took it to 26.7 us.
+  __device__ __forceinline__ double hessian_job(int job, double x, double y, double z, double u, double mu,
+                                                double& off) const {
+    const double mu2 = 1.0 - mu;
+    const bool acc = job >= 3;
+    const int k = acc ? job - 3 : job;
+    const double m = acc ? mu : mu2;
+    const double tt = x + (acc ? -mu2 : mu);  // x + mu | x - mu2
+    // job 0: t1^2, 1: y^2, 2: mu2 t1, 3: t2^2, 4: z^2, 5: mu t2
+    const double sq = (k == 0 ? tt : (job == 1 ? y : (job == 4 ? z : m))) * (job == 1 ? y : (job == 4 ? z : tt));
+    const double ts = from(sq, acc ? 3 : 0);
+    const double ys = from(sq, 1), zs = from(sq, 4);
+    const double t2s = from(sq, 3);
+    const double rr = (ts + ys) + zs;
+    const double den = hg_power_of_r2(rr, k == 2);  // r^3, on jobs 2 and 5 r^5
+    const double num[2] = {k == 1 ? y : m, k == 0 ? tt : (k == 1 ? z : sq)};
+    double q[2];
+    hg_quotients(num, den, q);
+    //            jobs 0..2 read   job 3          job 4          job 5
+    // s1         0: mu2/r3        2: mu2 t1/r5   5: mu/R5       2: mu2 t1/r5
+    // s2         3: mu/R3         5: mu t2/R5    2: mu2/r5      5: mu t2/R5
+    // f1         2: mu2/r5        0: t1/r3       1: y/r3        4: z/R3
+    // f2         5: mu/R5         3: t2/R3       4: y/R3        1: z/r3
+    const double s1 = from(job == 2 ? q[1] : q[0], nibble(0x252000u, job));
+    const double s2 = from(job == 5 ? q[1] : q[0], nibble(0x525333u, job));
+    const double f1 = from(job == 0 || job == 4 ? q[1] : q[0], nibble(0x410222u, job));
+    const double f2 = from(job == 1 || job == 3 ? q[1] : q[0], nibble(0x143555u, job));
+    // jobs 0..2: mu2/r5 3; the Coriolis term 2 vy, -2 vx on jobs 3, 4
+    const double a = (acc ? (job == 4 ? -2.0 : 2.0) : f1) * (acc ? u : 3.0);
+    // jobs 0..2: mu/R5 3; jobs 3..5: 3y, 3y, 3z of the off-diagonal entry
+    const double b = (acc ? (job == 5 ? z : y) : f2) * 3.0;
+    const double s = s1 + s2;
+    double P, A, U, B, W, C;
+    if (!acc) {
+      P = job == 2 ? -0.0 : 1.0;
+      A = a;
+      U = job == 0 ? ts : (job == 1 ? ys : zs);
+      B = b;
+      W = job == 0 ? t2s : (job == 1 ? ys : zs);
+      C = -s;
+    } else {
+      P = job == 3 ? x : (job == 4 ? y : -0.0);
+      A = job == 5 ? -mu : -mu2;
+      U = f1;
+      B = job == 5 ? -mu2 : -mu;
+      W = f2;
+      C = job == 5 ? -0.0 : a;
+    }
+    const double form = ((P + A * U) + B * W) + C;
+    // one product ((3a) b) c: (3y)(s) | ((3y) z)(s) | (3z)(s) (c = 1.0 exact)
+    off = (b * (job == 4 ? z : s)) * (job == 4 ? s : 1.0);
+    return form;
   }
 };
 

@@ -107,15 +107,6 @@ HG_XHD double hgp_exp(const HgLog2& g, uint64_t Y, bool neg, bool& ok) {
   return hgx_make((uint32_t)(bits >> 32), (uint32_t)bits);
 }
 
-// RN(x^1.5), or RN(x^2.5) when want25; y as for hgx_sqrt.  With x = m 2^e and
-// sqrt(x) = s 2^k (1 <= m, s < 2), the significand is that of m s or m^2 s:
-//   W: m in 64 bits (exact), or m^2's upper 64 (off by at most 1, centred);
-//   S: s in 64 bits from the root's 53 and its remainder (off by at most
-//     2048 * 3.4e-4 + 0.5 < 1.2);
-//   R = W S / 2^64 normalised to [2^63, 2^64): off by at most 2 (1.2 + 0.5) =
-//     3.4 units (x^1.5), 2 (1.2 + 1 + 0.5) = 5.4 (x^2.5).
-// Closer than that to a rounding boundary (one value in 256 and in 170) `ok`
-// is cleared.
 // sqrt(x)'s significand s in 64 bits.
 HG_XHD uint64_t hgp_root64(double x, float y) {
   uint64_t S_raw;
@@ -142,6 +133,15 @@ HG_XHD double hgp_make_power(double x, uint64_t R, bool want25, uint32_t sm, uin
 // |e| < 100: the powers stay far from the ends of the range
 HG_XHD bool hgp_power_range(double x) { return (hgx_hi(x) - (923u << 20)) < (200u << 20); }
 
+// RN(x^1.5), or RN(x^2.5) when want25; y as for hgx_sqrt.  With x = m 2^e and
+// sqrt(x) = s 2^k (1 <= m, s < 2), the significand is that of m s or m^2 s:
+//   W: m in 64 bits (exact), or m^2's upper 64 (off by at most 1, centred);
+//   S: s in 64 bits from the root's 53 and its remainder (off by at most
+//     2048 * 3.4e-4 + 0.5 < 1.2);
+//   R = W S / 2^64 normalised to [2^63, 2^64): off by at most 2 (1.2 + 0.5) =
+//     3.4 units (x^1.5), 2 (1.2 + 1 + 0.5) = 5.4 (x^2.5).
+// Closer than that to a rounding boundary (one value in 256 and in 170) `ok`
+// is cleared.
 HG_XHD double hgp_pow15_or_25(double x, float y, bool want25, bool& ok) {
   const uint64_t S = hgp_root64(x, y), m = hgp_significand64(x);
   uint64_t mm = hgp_mulhi64(m, m);
