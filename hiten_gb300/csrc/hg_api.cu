@@ -24,7 +24,7 @@ struct hg_handle {
   int* counters = nullptr;  // scratch: lane-refill counters
   int block = 32;           // threads per block (32, 64 or 128)
   int lanes_d6 = 0;         // lanes per 6-dim DOP853 trajectory: 0 auto, 1, 2, 6
-  int lanes_d42 = 0;        // lanes per 42-dim trajectory: 0 auto, 7, 14, 12 (paired warps, fixed RK)
+  int lanes_d42 = 0;        // lanes per 42-dim trajectory: 0 auto, 7, 14, 12 (paired warps), 18 (three warps, DOP853 four)
   int sm_capacity_x10 = 30;  // warps' FP64 demand an SM serves at full speed, x10 (layout cost models)
   long long refine_pool_max = 8LL << 30;  // largest record pool a single-pass call allocates (bytes)
   int seg_steps = 16;       // attempted steps per segment of the scheduled DOP853 driver
@@ -150,15 +150,17 @@ int lanes_d42_free(const hg_handle* h, int n) {
   return hg_internal::lanes_d42_free(n, h->sm_count, 0.1 * h->sm_capacity_x10);
 }
 
-// Paired-warp DOP853 launch (42-dim, no event, single pass): blocks of one
-// pair (two with HG_TUNE_BLOCK_THREADS 128).
-int launch_dop853_trio(hg_handle* h, const hg::DopParams& p, cudaStream_t s) {
+// Four-warp DOP853 launch (42-dim, no event, single pass): one block of 128
+// threads per five trajectories.
+int launch_dop853_quad(hg_handle* h, const hg::DopParams& p, cudaStream_t s) {
   const int grid = (p.N + hg::kPairTraj - 1) / hg::kPairTraj;
   if (grid < 1) return HG_OK;
-  hg::dop853_trio_kernel<<<grid, 96, hg::trio_dop_smem(), s>>>(p);
-  return check_launch(h, "dop853_trio_kernel");
+  hg::dop853_quad_kernel<<<grid, 128, hg::quad_dop_smem(), s>>>(p);
+  return check_launch(h, "dop853_quad_kernel");
 }
 
+// Paired-warp DOP853 launch: blocks of one pair (two with
+// HG_TUNE_BLOCK_THREADS 128).
 int launch_dop853_pair(hg_handle* h, const hg::DopParams& p, cudaStream_t s) {
   const int block = h->block >= 128 ? 128 : 64;
   const int per_block = (block / 64) * hg::kPairTraj;
@@ -695,7 +697,7 @@ int hg_propagate_dop853(hg_handle* h, double mu, int dim, int N, const double* y
     if (g == 12 && p.ev_index < 0)
       rc2 = launch_dop853_pair(h, p, s);
     else if (g == 18 && p.ev_index < 0)
-      rc2 = launch_dop853_trio(h, p, s);
+      rc2 = launch_dop853_quad(h, p, s);
     else
       rc2 = g == 14 ? launch_dop853<14>(h, p, s) : launch_dop853<7>(h, p, s);
   }
@@ -841,7 +843,7 @@ int hg_set_tuning(hg_handle* h, int key, int value) {
       return HG_OK;
     case HG_TUNE_LANES_D42:
       if (value != 0 && value != 7 && value != 14 && value != 12 && value != 18)
-        return fail(h, HG_ERR_ARGS, "lanes must be 0 (auto), 7, 14, 12 (paired warps) or 18 (three warps)");
+        return fail(h, HG_ERR_ARGS, "lanes must be 0 (auto), 7, 14, 12 (paired warps) or 18 (three or four warps)");
       h->lanes_d42 = value;
       return HG_OK;
     case HG_TUNE_SPREAD:

@@ -682,11 +682,11 @@ void stm_leg(const Ws& w, double mu, const hg_newton_opts& o, int sms, cudaStrea
   p.ws_prev_pow = w.wpp;
   p.ws_q = w.wq;
   if constexpr (G == 12 || G == 18) {
-    // the paired (12) and three-warp (18) layouts: five trajectories per
+    // the paired (12) and four-warp (18) layouts: five trajectories per
     // block, the live count read from n_in (their list is the identity)
     const int grid = (w.cap + hg::kPairTraj - 1) / hg::kPairTraj;
     if constexpr (G == 18)
-      hg::dop853_trio_kernel<<<grid, 96, hg::trio_dop_smem(), s>>>(p);
+      hg::dop853_quad_kernel<<<grid, 128, hg::quad_dop_smem(), s>>>(p);
     else
       hg::dop853_pair_kernel<<<grid, 64, hg::pair_dop_smem(64), s>>>(p);
   } else {
@@ -706,7 +706,7 @@ int lanes_d6(int n, int sms, int tuned) {
 }
 
 // STM leg layout: the handle's tuning, else the rule of event-free 42-dim runs
-// (2048 orbits: trio 17.0 ms, pair 19.1; 4096: 27.7 and 25.1).
+// (2048 orbits: four warps 16.3 ms, pair 18.9; 4096: 24.6 and 24.7).
 int lanes_d42(int tuned, int n, int sms) {
   if (tuned == 7 || tuned == 14 || tuned == 12 || tuned == 18) return tuned;
   return hg_internal::lanes_d42_free(n, sms, 3.0);

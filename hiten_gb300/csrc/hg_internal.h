@@ -53,15 +53,15 @@ inline int lanes_d6(long long n, int sms, double sm_capacity) {
   return best;
 }
 
-// Layout of an event-free single-pass 42-dim run of n trajectories: three warps
-// per five of them (18) while an SM holds at most three such groups, warp pairs
-// (12) beyond.  Measured on GB300 (us per step; G = 7 and 14 are behind at
-// every size):
-//   n              700    1000   1500   2048   4096   8192
-//   RK8, trio      28.9   32.6   32.6   42.4   77.4   142
-//   RK8, pair      40.4   40.6   40.6   43.3   74.2   155
-//   DOP853, trio   37.8   41.9   42.2   54.3   131    197
-//   DOP853, pair   52.0   52.6   52.7   56.2   91.1   180
+// Layout of an event-free single-pass 42-dim run of n trajectories: 18 (three
+// warps per five of them, four for DOP853) while an SM holds at most three such
+// groups, warp pairs (12) beyond.  Measured on GB300 (us per step; G = 7 and 14
+// are behind at every size):
+//   n               760    1024   1500   2048   4096   8192
+//   RK8, 18         26.9   30.6   30.6   41.2   76.4   140
+//   RK8, pair       41.4   41.7   41.6   44.1   72.5   159
+//   DOP853, 18      34.1   40.6   40.5   53.1   104    204
+//   DOP853, pair    51.7   52.1   52.2   55.9   90.2   178
 inline int lanes_d42_free(long long n, int sms, double sm_capacity) {
   const double groups = (double)((n + 4) / 5);
   return groups <= sm_capacity * sms ? 18 : 12;

@@ -292,14 +292,12 @@ struct PairStm {
   }
 };
 
-// Half-column STM warps of the three-warp layout (dop853_trio_kernel): two
+// Half-column STM warps of the three-warp layout (fixed_rk_trio_kernel): two
 // warps share the 36 STM components of five trajectories.  A half-group of
 // six lanes holds three columns of one trajectory (columns 3 half .. 3 half +
 // 2), each column on a lane pair as in Layout<14>: the even lane rows 0..2,
 // the odd lane rows 3..5; warp w holds half-groups 5w .. 5w + 4 (trajectory
-// = half-group / 2, half = half-group % 2).  A half-group is a complete
-// six-lane group for the step control (coefficients, norms, step-size
-// factor), so each trajectory's two halves take the same decisions.
+// = half-group / 2, half = half-group % 2).
 struct PairStmHalf {
   using Ops = FusedOps;
   Ops ops;
@@ -312,7 +310,6 @@ struct PairStmHalf {
   PairLink* link;
   mutable unsigned seq;
   mutable bool broken;
-  __device__ __forceinline__ int flag_slot() const { return 43 + half; }
   __device__ __forceinline__ int comp(int r) const {
     const int r6 = role % 6;
     return 6 * (3 * (r6 & 1) + r) + 3 * half + (r6 >> 1);
@@ -354,6 +351,64 @@ struct PairStmHalf {
     dv[0] = neg_if(d0, comp(0) >= dir.neg_lo && comp(0) < dir.neg_hi);
     dv[1] = neg_if(d1, comp(1) >= dir.neg_lo && comp(1) < dir.neg_hi);
     dv[2] = neg_if(d2, comp(2) >= dir.neg_lo && comp(2) < dir.neg_hi);
+  }
+};
+
+// Third-column STM warps of the four-warp layout: three warps share the 36 STM
+// components of five trajectories.  A third-group of six lanes holds two
+// columns of one trajectory, each on three lanes: lane i of a column holds its
+// rows i and 3 + i.  The derivative of row i is the lane's own row 3 + i, and
+// lane i forms row 3 + i of F(x) Phi[:, c] from rows 0..2 (its own and the two
+// other lanes') and its row of the Hessian: six FP64 instructions a
+// right-hand side where the half column's lanes take eleven.  Warp w holds
+// third-groups 5w .. 5w + 4 (trajectory = third-group / 3).  A third-group is a
+// complete six-lane group for the step control (coefficients, norms, step-size
+// factor), so a trajectory's three parts take the same decisions.
+struct PairStmThird {
+  using Ops = FusedOps;
+  Ops ops;
+  static constexpr int D = 42;
+  static constexpr int NC = 2;
+  static constexpr bool kState = false;
+  int t, part;     // part 0..2: columns 2 part, 2 part + 1
+  int role, base;  // lane placement within the third-group (6, 7 on the shadow lanes)
+  unsigned gmask;
+  PairLink* link;
+  mutable unsigned seq;
+  mutable bool broken;
+  __device__ __forceinline__ int flag_slot() const { return 43 + part; }
+  __device__ __forceinline__ int row() const { return role % 3; }
+  __device__ __forceinline__ int comp(int r) const { return 6 * (3 * r + role % 3) + 2 * part + (role % 6) / 3; }
+  __device__ __forceinline__ double from(double v, int r) const { return __shfl_sync(gmask, v, r); }
+  __device__ __forceinline__ void rhs(const double (&v)[2], double mu, const Dir& dir, double (&dv)[2]) const {
+    (void)mu;
+    const unsigned b = seq % kPairSlots;
+    const int i = row();
+    const int col = base + (role % 6) / 3 * 3;  // first lane of the column
+    // rows 0..2 of the column, the paired velocity (row 3 takes 2 v4, row 4 -2 v3)
+    const double p0 = from(v[0], col), p1 = from(v[0], col + 1), p2 = from(v[0], col + 2);
+    const double w = from(v[1], col + (i == 0 ? 1 : 0));
+    // this lane's row of the Hessian (xx, yy, zz, xy, yz, xz)
+    double h0 = 0.0, h1 = 0.0, h2 = 0.0;
+    if (!broken) {
+      const bool ok = mbar_wait(&link->full[b], (seq / kPairSlots) & 1u);
+      broken = !__all_sync(0xFFFFFFFFu, ok);
+    }
+    if (!broken) {
+      const double* e = link->H[b][t];
+      h0 = e[i == 0 ? 0 : (i == 1 ? 3 : 5)];
+      h1 = e[i == 0 ? 3 : (i == 1 ? 1 : 4)];
+      h2 = e[i == 0 ? 5 : (i == 1 ? 4 : 2)];
+      mbar_arrive(&link->empty[b]);
+    }
+    ++seq;
+    const Ops& o = ops;
+    const double s = o.add(o.add(o.mul(h0, p0), o.mul(h1, p1)), o.mul(h2, p2));
+    // (the doubled velocities are exact: one rounding)
+    const double c = fma(i == 0 ? 2.0 : -2.0, w, s);
+    const double d1 = i == 2 ? s : c;
+    dv[0] = neg_if(v[1], comp(0) >= dir.neg_lo && comp(0) < dir.neg_hi);
+    dv[1] = neg_if(d1, comp(1) >= dir.neg_lo && comp(1) < dir.neg_hi);
   }
 };
 
@@ -474,7 +529,7 @@ __global__ void __launch_bounds__(128) fixed_rk_pair_kernel(FixedParams p) {
 
 // Three-warp fixed-step RK (42-dim, no event): blocks of 96 threads, warp 0
 // the state warp of five trajectories, warps 1 and 2 their STM as half
-// columns (PairStmHalf), as dop853_trio_kernel lays them out.  The STM
+// columns (PairStmHalf).  The STM
 // warp's stage work is halved and a batch of N trajectories issues 3N / 5
 // warps instead of 2N / 5: faster while every SM holds at most one group
 // (below about 760 trajectories), level or slower beyond, where two groups'
@@ -559,8 +614,8 @@ __global__ void __launch_bounds__(96) fixed_rk_trio_kernel(FixedParams p) {
 // hand-off has all 32 lanes of both warps.
 struct PairGather {
   // slot, trajectory, vector, 42 components + flags: [42] the state warp's,
-  // [43], [44] the STM's (one warp: both; two half-column warps: one each)
-  double v[2][kPairTraj][2][45];
+  // [43..45] the STM's (one warp: all; three third-column warps: one each)
+  double v[2][kPairTraj][2][46];
   unsigned long long bar[2];
 };
 
@@ -580,7 +635,7 @@ __device__ __forceinline__ void pair_exchange(const LT& L, PairGather* gx, unsig
       }
       if (L.role == 0) {
         va[L.flag_slot()] = flag;
-        if constexpr (LT::kState == false && LT::NC == 6) va[44] = flag;
+        if constexpr (!LT::kState && LT::NC == 6) va[44] = va[45] = flag;
       }
     }
     mbar_arrive(&gx->bar[sl]);
@@ -589,7 +644,7 @@ __device__ __forceinline__ void pair_exchange(const LT& L, PairGather* gx, unsig
   }
   ++gseq;
   dots42_group(L, va, vb, dot_a, dot_b);
-  flag_all = (va[42] != 0.0 && va[43] != 0.0 && va[44] != 0.0) ? 1.0 : 0.0;
+  flag_all = (va[42] != 0.0 && va[43] != 0.0 && va[44] != 0.0 && va[45] != 0.0) ? 1.0 : 0.0;
 }
 
 // Shared memory of a warp: stage derivatives, then its groups' products.
@@ -601,15 +656,15 @@ __host__ __device__ constexpr size_t pair_dop_bytes() {
   return sizeof(PairLink) + sizeof(PairGather) + (pair_dop_doubles(1) + pair_dop_doubles(6)) * sizeof(double);
 }
 __host__ __device__ constexpr size_t pair_dop_smem(int block) { return (size_t)(block / 64) * pair_dop_bytes(); }
-__host__ __device__ constexpr size_t trio_dop_smem() {
-  return (size_t)(pair_dop_doubles(1) + 2 * pair_dop_doubles(3)) * sizeof(double);
+__host__ __device__ constexpr size_t quad_dop_smem() {
+  return (size_t)(pair_dop_doubles(1) + 3 * pair_dop_doubles(2)) * sizeof(double);
 }
 
 // One warp's part of the DOP853 propagation of its five trajectories.
 // Decisions that set how many hand-offs a step makes (keep stepping, build a
 // dense cache) are votes over the warp (BLOCK = false: both warps of a pair
-// hold the same trajectories) or over the block (BLOCK = true: the three
-// warps of a trio hold different subsets).  Returns its broken flag.
+// hold the same trajectories) or over the block (BLOCK = true: the four
+// warps of a quad hold different subsets).  Returns its broken flag.
 template <bool BLOCK, class LT>
 __device__ __forceinline__ bool pair_dop_run(const LT& L, const DopParams& p, PairGather* gx, double* sm, int traj,
                                              bool valid, bool writes) {
@@ -837,22 +892,26 @@ static __global__ void __launch_bounds__(128, 3) dop853_pair_kernel(DopParams p)
   if (!stm && valid && pl.role == 0 && p.status && (broken || lk->broken)) p.status[traj] = HG_SYNC_TIMEOUT;
 }
 
-// Three-warp DOP853 (42-dim, single pass, no event): blocks of 96 threads,
-// warp 0 the state warp of five trajectories, warps 1 and 2 their STM as
-// half-columns (PairStmHalf) -- the STM warp's stage work halved, for
-// batches too small to fill the GPU, where one warp's step sets the time.
-// The Hessian ring's "empty" barriers take both STM warps' arrivals, the
-// norm gather all three warps'.
-static __global__ void __launch_bounds__(96) dop853_trio_kernel(DopParams p) {
+// Four-warp DOP853 (42-dim, single pass, no event): blocks of 128 threads,
+// warp 0 the state warp of five trajectories, warps 1 to 3 their STM as thirds
+// of columns (PairStmThird): two components a lane in the stage sums, the
+// error norms and the quotients, where half columns on two warps hold three.
+// A step of up to 760 trajectories took 36.4 us on three warps and takes 33.8;
+// 1000 to 2048 trajectories (two or three groups an SM) are level, 40.4 and
+// 53.  (Fixed steps, with neither norms nor quotients, keep half columns: 26.8 us
+// a step on three warps, 28.1 on four, whose fourth warp only takes turns at
+// the FP64 unit.)  The Hessian ring's "empty" barriers take the three STM warps'
+// arrivals, the norm gather all four warps'.
+static __global__ void __launch_bounds__(128) dop853_quad_kernel(DopParams p) {
   __shared__ PairLink link;
   __shared__ PairGather gather;
-  extern __shared__ double sm_step[];  // trio_dop_smem()
+  extern __shared__ double sm_step[];  // quad_dop_smem()
   const int w = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   if (threadIdx.x < (int)kPairSlots) {
     mbar_init(&link.full[threadIdx.x], 32);
-    mbar_init(&link.empty[threadIdx.x], 64);
-    if (threadIdx.x < 2) mbar_init(&gather.bar[threadIdx.x], 96);
+    mbar_init(&link.empty[threadIdx.x], 96);
+    if (threadIdx.x < 2) mbar_init(&gather.bar[threadIdx.x], 128);
     if (threadIdx.x == 0) link.broken = 0;
   }
   __syncthreads();
@@ -862,8 +921,8 @@ static __global__ void __launch_bounds__(96) dop853_trio_kernel(DopParams p) {
   const int N = p.n_in ? *p.n_in : p.N;
   const bool active = group * kPairTraj < N;  // uniform over the block
   // trajectory of this lane within the group
-  const int hg = 5 * (w - 1) + pl.t;                 // STM warps: half-group 0..9
-  const int tg = w == 0 ? pl.t : hg / 2;
+  const int tp = 5 * (w - 1) + pl.t;  // STM warps: third-group 0..14
+  const int tg = w == 0 ? pl.t : tp / 3;
   const int traj = group * kPairTraj + tg;
   const bool valid = active && traj < N;
   const int tc = valid ? traj : (active ? N - 1 : 0);
@@ -880,16 +939,16 @@ static __global__ void __launch_bounds__(96) dop853_trio_kernel(DopParams p) {
       L.broken = false;
       broken = pair_dop_run<true>(L, p, &gather, sm_step, tc, valid, valid && pl.role < 6);
     } else {
-      PairStmHalf L;
+      PairStmThird L;
       L.t = tg;
-      L.half = hg & 1;
+      L.part = tp % 3;
       L.role = pl.role;
       L.base = pl.base;
       L.gmask = pl.gmask;
       L.link = &link;
       L.seq = 0;
       L.broken = false;
-      broken = pair_dop_run<true>(L, p, &gather, sm_step + pair_dop_doubles(1) + (w - 1) * pair_dop_doubles(3), tc, valid,
+      broken = pair_dop_run<true>(L, p, &gather, sm_step + pair_dop_doubles(1) + (w - 1) * pair_dop_doubles(2), tc, valid,
                                   valid && pl.role < 6);
       if (broken && lane == 0) link.broken = 1;
     }
