@@ -133,9 +133,13 @@ struct PairLane {
   }
 };
 
-// State warp: one state component per lane (NC = 1).
+// State warp: one state component per lane (NC = 1).  Its stage sums are plain
+// in the layouts whose chain it is, and three-register multiply-adds (OPS) beside
+// one STM warp, where a filled SM's FP64 unit sets the time: 8192 trajectories,
+// RK8 159 -> 150 us a step, DOP853 178 -> 176.
+template <class OPS>
 struct PairState {
-  using Ops = PlainOps;
+  using Ops = OPS;
   Ops ops;
   static constexpr int D = 42;
   static constexpr int NC = 1;
@@ -491,7 +495,7 @@ __global__ void __launch_bounds__(128) fixed_rk_pair_kernel(FixedParams p) {
   bool finite = true, broken = false;
   if (active) {
     if (!stm) {
-      PairState L;
+      PairState<FusedOps> L;
       L.role = pl.role;
       L.base = pl.base;
       L.t = pl.t;
@@ -564,7 +568,7 @@ __global__ void __launch_bounds__(96) fixed_rk_trio_kernel(FixedParams p) {
   bool finite = true, broken = false;
   if (active) {
     if (w == 0) {
-      PairState L;
+      PairState<PlainOps> L;
       L.role = pl.role;
       L.base = pl.base;
       L.t = pl.t;
@@ -864,7 +868,7 @@ static __global__ void __launch_bounds__(128, 3) dop853_pair_kernel(DopParams p)
   bool broken = false;
   if (active) {
     if (!stm) {
-      PairState L;
+      PairState<FusedOps> L;
       L.role = pl.role;
       L.base = pl.base;
       L.t = pl.t;
@@ -929,7 +933,7 @@ static __global__ void __launch_bounds__(128) dop853_quad_kernel(DopParams p) {
   bool broken = false;
   if (active) {
     if (w == 0) {
-      PairState L;
+      PairState<PlainOps> L;
       L.role = pl.role;
       L.base = pl.base;
       L.t = pl.t;
