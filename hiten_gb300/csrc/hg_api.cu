@@ -6,11 +6,11 @@
 // allocation is counted (HG_COUNTER_ALLOCATIONS).
 #include <cuda_runtime.h>
 
-#include <algorithm>
 #include <stdarg.h>
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <new>
 
 #include "hg_internal.h"
@@ -301,7 +301,8 @@ int launch_refine(hg_handle* h, hg::DopParams p, cudaStream_t s) {
 
 int refine_pending(hg_handle* h, const hg::DopParams& p, int dim, cudaStream_t s) {
   if (!p.rec) return HG_OK;
-  return dim == 6 ? launch_refine<1>(h, p, s) : launch_refine<7>(h, p, s);
+  if (dim != 6) return launch_refine<7>(h, p, s);
+  return hg_internal::refine_lanes(p.rec_ld, h->sm_count) == 6 ? launch_refine<6>(h, p, s) : launch_refine<1>(h, p, s);
 }
 
 // Grow-only device buffer of the handle: a no-op (no allocation) when it

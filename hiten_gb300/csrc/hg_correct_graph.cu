@@ -574,6 +574,17 @@ int resident_blocks(K kern, int block, int sms, size_t smem = 0) {
   return per_sm * sms;
 }
 
+// Refinement of the event leg's saved crossings (records [0, refine_count)).
+template <int G>
+void refine_leg(hg::DopParams p, int sms, cudaStream_t s) {
+  constexpr int kTpw = hg::Layout<G>::TPW;
+  const int need = (int)((p.rec_ld + kTpw - 1) / kTpw);
+  const int cap = resident_blocks(hg::refine_kernel<G>, 32, sms);
+  const int grid = need < cap ? need : cap;
+  p.stride = grid * kTpw;
+  hg::refine_kernel<G><<<grid, 32, 0, s>>>(p);
+}
+
 // The event leg on trial slots [0, sc[0]): DOP853 in list mode with the
 // undirected y = 0 event, then the lock-step refinement of the crossings.
 template <int G>
@@ -632,13 +643,10 @@ void event_leg(const Ws& w, double mu, const hg_newton_opts& o, int sms, cudaStr
   const int grid = need < cap_blocks ? need : cap_blocks;
   p.stride = grid * tpb;
   hg::dop853_kernel<G, false><<<grid, 32, hg::dop_smem_bytes<G>(32), s>>>(p);
-  // refinement of the saved crossings (records [0, refine_count))
-  const int rneed = (int)((capr + 31) / 32);
-  const int rcap = resident_blocks(hg::refine_kernel<1>, 32, sms);
-  const int rgrid = rneed < rcap ? rneed : rcap;
-  hg::DopParams q = p;
-  q.stride = rgrid * 32;
-  hg::refine_kernel<1><<<rgrid, 32, 0, s>>>(q);
+  if (hg_internal::refine_lanes(capr, sms) == 6)
+    refine_leg<6>(p, sms, s);
+  else
+    refine_leg<1>(p, sms, s);
   gc_trial_residual<<<ctl < 1 ? 1 : ctl, 256, 0, s>>>(w);
   *launches += 4;
 }

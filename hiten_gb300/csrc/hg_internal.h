@@ -67,4 +67,13 @@ inline int lanes_d42_free(long long n, int sms, double sm_capacity) {
   return groups <= sm_capacity * sms ? 18 : 12;
 }
 
+// Lanes per crossing of a deferred refinement of up to `records` 6-dim
+// crossings.  Six lanes halve the latency (a component of the dense cache a
+// lane, two halvings a pass), one lane takes fewer FP64 instructions a
+// crossing.  Measured on GB300 (us, 152 SMs; the lines meet at 43 an SM):
+//   records    50    400   1237   2500   4000   6000   8000   16384
+//   one lane   82.8  74.7  74.6   74.3   74.0   74.6   74.7   80.7
+//   six lanes  33.5  34.1  34.8   38.2   52.4   66.8   90.0   183
+inline int refine_lanes(long long records, int sms) { return records <= 40LL * sms ? 6 : 1; }
+
 }  // namespace hg_internal

@@ -1933,7 +1933,9 @@ struct EvCtx {
 
 // _dop853_refine_in_step: bisection for the crossing on the step's dense
 // interpolant (rows F, step size h, g at the step start g_left); returns the
-// crossing as a fraction x of the step.
+// crossing as a fraction x of the step.  G = 6: three lanes evaluate a midpoint
+// and both midpoints that can follow it, so a pass over the interpolant's sixteen
+// serial FP64 instructions decides two halvings.
 template <int G>
 __device__ __forceinline__ double refine_in_step(const EvCtx<G>& ev, const double (&y)[Layout<G>::NC],
                                                  const double (&F)[7][Layout<G>::NC], double h, double g_left,
@@ -1942,9 +1944,42 @@ __device__ __forceinline__ double refine_in_step(const EvCtx<G>& ev, const doubl
   double fe[7];
 #pragma unroll
   for (int i = 0; i < 7; ++i) fe[i] = pick<NC>(F[i], ev.r);
-  const double ye = pick<NC>(y, ev.r);
+  double ye = pick<NC>(y, ev.r);
   double a = 0.0, b = 1.0;
   double x_hit = -1.0;
+  if constexpr (G == 6) {
+    const int lane = threadIdx.x & 31, third = lane % 3, base = lane - lane % 6;
+#pragma unroll
+    for (int i = 0; i < 7; ++i) fe[i] = ev.bcast(fe[i]);
+    ye = ev.bcast(ye);
+    bool done = false;
+    for (int it = 0; it < 128 && !done; it += 2) {
+      const double m0 = 0.5 * (a + b);
+      const double node = 0.5 * ((third == 2 ? m0 : a) + (third == 1 ? m0 : b));
+      const double g = DopLane<G>::eval_row(ye, fe, node) - p.ev_offset;
+      double g_mid = __shfl_sync(ev.gmask, g, base);
+      const double g_low = __shfl_sync(ev.gmask, g, base + 1), g_high = __shfl_sync(ev.gmask, g, base + 2);
+      double mid = m0;
+      for (int s = 0; s < 2 && !done; ++s) {
+        if (fabs(g_mid) <= p.gtol) {
+          x_hit = mid;
+          done = true;
+        } else {
+          const bool crossed = crossed_direction(g_left, g_mid, p.ev_dir);
+          if (crossed) {
+            b = mid;
+          } else {
+            a = mid;
+            g_left = g_mid;
+          }
+          done = (b - a) * fabs(h) <= p.xtol;
+          mid = 0.5 * (a + b);
+          g_mid = crossed ? g_low : g_high;
+        }
+      }
+    }
+    return x_hit < 0.0 ? b : x_hit;
+  }
   for (int it = 0; it < 128; ++it) {
     const double mid = 0.5 * (a + b);
     const double g_mid = ev.bcast(ev.mine ? (DopLane<G>::eval_row(ye, fe, mid) - p.ev_offset) : 0.0);

@@ -443,7 +443,9 @@ struct hg_server {
                        : segment<1>(p, live, sms, s);
         else
           e = g == 14 ? segment<14>(p, live, sms, s) : segment<7>(p, live, sms, s);
-        if (e == cudaSuccess && k.has_ev) e = d == 6 ? refine<1>(p, sms, s) : refine<7>(p, sms, s);
+        if (e == cudaSuccess && k.has_ev)
+          e = d != 6 ? refine<7>(p, sms, s)
+                     : (hg_internal::refine_lanes(p.rec_ld, sms) == 6 ? refine<6>(p, sms, s) : refine<1>(p, sms, s));
         if (e != cudaSuccess) return HG_ERR_CUDA;
         // finished slots of this segment's list: rows gathered into staging half h
         const int blocks = std::min((live + 255) / 256, 1024);
