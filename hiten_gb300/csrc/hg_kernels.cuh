@@ -1,12 +1,16 @@
 // sm_103a kernels for the CR3BP propagation path (FP64 throughout).
 //
 // Execution model.  GB300 issues FP64 at a small fraction of its FP32 rate,
-// so the kernels are bound by the FP64 pipe, not by HBM: state and Runge-
-// Kutta stages live in registers, HBM sees only initial states, sampled
-// outputs and saved event steps.  Lane layouts (Layout<G>):
+// so the kernels are bound by the FP64 pipe, not by HBM: the state lives in
+// registers, the Runge-Kutta stages in registers or shared memory, and HBM sees
+// only initial states, sampled outputs and saved event steps.  What can leave
+// the FP64 unit does: roots, quotients and powers are formed on the FP32 and
+// integer pipes (hg_exact.cuh, hg_powint.cuh).  Lane layouts (Layout<G>):
 //   * G = 1  (6-dim state): one lane owns one trajectory.
 //   * G = 2  (6-dim): a lane pair (position / velocity halves).
 //   * G = 6  (6-dim): six lanes, one component each.
+//   * G = 30 (6-dim): five copies of the six-lane group, a warp per trajectory;
+//            the copies share out the stage sums.
 //   * G = 7  (42-dim state + STM): a group of 7 lanes owns one trajectory;
 //            lane j < 6 holds STM column j (components 6r+j, r = 0..5), lane 6
 //            holds the state (components 36..41).  Column j of dPhi = F(x)Phi
@@ -1978,25 +1982,24 @@ __device__ __forceinline__ double refine_in_step(const EvCtx<G>& ev, const doubl
         }
       }
     }
-    return x_hit < 0.0 ? b : x_hit;
-  }
-  for (int it = 0; it < 128; ++it) {
-    const double mid = 0.5 * (a + b);
-    const double g_mid = ev.bcast(ev.mine ? (DopLane<G>::eval_row(ye, fe, mid) - p.ev_offset) : 0.0);
-    if (fabs(g_mid) <= p.gtol) {
-      x_hit = mid;
-      break;
+  } else {
+    for (int it = 0; it < 128; ++it) {
+      const double mid = 0.5 * (a + b);
+      const double g_mid = ev.bcast(ev.mine ? (DopLane<G>::eval_row(ye, fe, mid) - p.ev_offset) : 0.0);
+      if (fabs(g_mid) <= p.gtol) {
+        x_hit = mid;
+        break;
+      }
+      if (crossed_direction(g_left, g_mid, p.ev_dir)) {
+        b = mid;
+      } else {
+        a = mid;
+        g_left = g_mid;
+      }
+      if ((b - a) * fabs(h) <= p.xtol) break;
     }
-    if (crossed_direction(g_left, g_mid, p.ev_dir)) {
-      b = mid;
-    } else {
-      a = mid;
-      g_left = g_mid;
-    }
-    if ((b - a) * fabs(h) <= p.xtol) break;
   }
-  if (x_hit < 0.0) x_hit = b;
-  return x_hit;
+  return x_hit < 0.0 ? b : x_hit;
 }
 
 // A crossing step saved for deferred refinement, structure of arrays with

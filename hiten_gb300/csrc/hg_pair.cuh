@@ -1,6 +1,6 @@
-// Paired-warp layout for the 42-dim variational system: fixed-step RK
-// (fixed_rk_pair_kernel) and single-pass DOP853 without an event
-// (dop853_pair_kernel).
+// Layouts of the 42-dim variational system on several warps: fixed-step RK
+// (fixed_rk_pair_kernel, fixed_rk_trio_kernel) and single-pass DOP853 without
+// an event (dop853_pair_kernel, dop853_quad_kernel).
 //
 // Why.  On GB300 a warp has one FP64 instruction in flight at a time, for
 // 64 cycles whatever the number of active lanes (76 when four warps share the
@@ -13,7 +13,7 @@
 //
 // Layout.  A trajectory group is five trajectories served by two warps:
 //   * the state warp: lane 6t + j (t < 5, j < 6) holds state component 36 + j
-//     of trajectory t and does job j of the shared Hessian (hessian_split);
+//     of trajectory t and does job j of the shared Hessian (hessian_job);
 //     lanes 30 and 31 shadow group 4 (they repeat job 0 and write nothing);
 //   * the STM warp: lane 6t + c holds column c of Phi (components 6r + c,
 //     r = 0..5); lanes 30 and 31 shadow column 5 of trajectory 4.
@@ -533,12 +533,11 @@ __global__ void __launch_bounds__(128) fixed_rk_pair_kernel(FixedParams p) {
 
 // Three-warp fixed-step RK (42-dim, no event): blocks of 96 threads, warp 0
 // the state warp of five trajectories, warps 1 and 2 their STM as half
-// columns (PairStmHalf).  The STM
-// warp's stage work is halved and a batch of N trajectories issues 3N / 5
-// warps instead of 2N / 5: faster while every SM holds at most one group
-// (below about 760 trajectories), level or slower beyond, where two groups'
-// six warps share an SM's FP64 unit.  The Hessian ring's "empty" barriers
-// take both STM warps' arrivals.
+// columns (PairStmHalf).  The STM warp's stage work is halved and a batch of N
+// trajectories issues 3N / 5 warps instead of 2N / 5: an RK8 step 26.8 us
+// against the pair's 41.4 while every SM holds one group, 30.6 / 41.7 with two,
+// 41.2 / 42.9 with three, behind beyond (the groups share an SM's FP64 unit).
+// The Hessian ring's "empty" barriers take both STM warps' arrivals.
 template <int ORDER>
 __host__ __device__ constexpr size_t trio_fixed_smem() {
   return (size_t)(pair_fixed_doubles<ORDER>(1) + 2 * pair_fixed_doubles<ORDER>(3)) * sizeof(double);
