@@ -37,6 +37,7 @@
 
 #include "hg_crmath.cuh"
 #include "hg_exact.cuh"
+#include "hg_fp64_ops.cuh"
 #include "hg_powint.cuh"
 #include "hg_tableaux.h"
 #include "hitengpu.h"
@@ -96,31 +97,6 @@ struct DopTab {
 __device__ __forceinline__ double neg_if(double v, bool neg) {
   return __longlong_as_double(__double_as_longlong(v) ^ (neg ? (long long)0x8000000000000000ull : 0ll));
 }
-
-// Products, sums and differences of a layout.  With four or more warps on an
-// SM its FP64 unit takes a multiply, an add, or a fused multiply-add with a
-// constant operand every 19.0 cycles, but a fused multiply-add of three
-// registers every 16.0 (measured, 4 to 32 warps); one warp alone waits 63.1 and
-// 64.6.  So the layouts that fill the unit form them as fused multiply-adds
-// with a neutral operand: a b + (-0), a 1 + b and (-b) 1 + a round once and have
-// the bits of a * b, a + b and a - b, signed zeros included.  The neutral
-// operands come by volatile loads: the compiler would fold known ones back.
-struct PlainOps {
-  __device__ __forceinline__ double mul(double a, double b) const { return a * b; }
-  __device__ __forceinline__ double add(double a, double b) const { return a + b; }
-  __device__ __forceinline__ double sub(double a, double b) const { return a - b; }
-};
-__device__ static double hg_neutral[2] = {1.0, -0.0};
-struct FusedOps {
-  double one, nz;
-  __device__ __forceinline__ FusedOps() {
-    asm volatile("ld.volatile.global.f64 %0, [%1];" : "=d"(one) : "l"(hg_neutral));
-    asm volatile("ld.volatile.global.f64 %0, [%1];" : "=d"(nz) : "l"(hg_neutral + 1));
-  }
-  __device__ __forceinline__ double mul(double a, double b) const { return fma(a, b, nz); }
-  __device__ __forceinline__ double add(double a, double b) const { return fma(a, one, b); }
-  __device__ __forceinline__ double sub(double a, double b) const { return fma(-b, one, a); }
-};
 
 // dynamics/rtbp.py:30-74 (_crtbp_accel), numba lowering of ** (x*x, x*(x*x)).
 // The distances and the six quotients over r1^3 and r2^3 are formed on the

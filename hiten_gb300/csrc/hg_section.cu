@@ -23,6 +23,7 @@
 #include <math.h>
 
 #include "hg_exact.cuh"
+#include "hg_fp64_ops.cuh"
 #include "hg_section_skip.cuh"
 #include "hitengpu.h"
 
@@ -422,8 +423,8 @@ __global__ void __launch_bounds__(kSecBlock) section_kernel(SecParams p) {
 // One thread per trajectory and chunk of samples; chunks so many that the
 // device is full (a manifold has tens to thousands of trajectories of thousands
 // of samples: one thread for all samples of each left 12 of 152 SMs busy and
-// took 16.3 ms for 1600 x 4713, 0.49 ms here).  Bound: the FP64 unit, 27
-// instructions a sample (0.33 ms); the two roots and quotients are on the integer pipes
+// took 16.3 ms for 1600 x 4713, 0.48 ms here; 0.49 with plain products and
+// sums).  Bound: the FP64 unit, 27 instructions a sample (0.33 ms); the two roots and quotients are on the integer pipes
 // (hg_exact.cuh), and what is monotone is taken once per trajectory: the root
 // of the least squared distance, the quotient of the largest |C - C0|.
 // The chunks' results meet in the outputs as integers: non-negative doubles
@@ -433,15 +434,19 @@ struct FilterSample {
   double C;       // Jacobi constant
 };
 
-__device__ __forceinline__ FilterSample filter_sample(const double* s, long long ld, double mu, double mu1) {
+__device__ __forceinline__ FilterSample filter_sample(const hg::FusedOps& o, const double* s, long long ld, double mu,
+                                                      double mu1) {
   FilterSample r;
   const double x = s[0], y = s[ld], z = s[2 * ld], vx = s[3 * ld], vy = s[4 * ld], vz = s[5 * ld];
-  const double a = x + mu, b = (x - 1.0) + mu, f = x - mu1;
-  const double yy = y * y, zz = z * z;
-  r.q1 = (a * a + yy) + zz;
-  r.q2 = (b * b + yy) + zz;
-  const double r1 = hg_sqrt(r.q1), r2 = hg_sqrt((f * f + yy) + zz);
-  r.C = ((x * x + yy) + 2.0 * (hg_div(mu1, r1) + hg_div(mu, r2))) - ((vx * vx + vy * vy) + vz * vz);
+  const double a = o.add(x, mu), b = o.add(o.add(x, -o.one), mu), f = o.sub(x, mu1);
+  const double yy = o.mul(y, y), zz = o.mul(z, z);
+  auto square_sum = [&](double u) { return o.add(o.add(o.mul(u, u), yy), zz); };
+  r.q1 = square_sum(a);
+  r.q2 = square_sum(b);
+  const double r1 = hg_sqrt(r.q1), r2 = hg_sqrt(square_sum(f));
+  // (the doubled sum is exact: one rounding)
+  r.C = o.sub(fma(o.add(hg_div(mu1, r1), hg_div(mu, r2)), 2.0, o.add(o.mul(x, x), yy)),
+              o.add(o.add(o.mul(vx, vx), o.mul(vy, vy)), o.mul(vz, vz)));
   return r;
 }
 
@@ -470,12 +475,13 @@ __global__ void __launch_bounds__(kFilterBlock) filters_kernel(int N, int m, int
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   const double mu1 = 1.0 - mu;
-  const FilterSample first = filter_sample(samples + i, ld, mu, mu1);
+  const hg::FusedOps o;
+  const FilterSample first = filter_sample(o, samples + i, ld, mu, mu1);
   unsigned long long q1 = pattern(first.q1), q2 = pattern(first.q2), e = 0;
   const int lo = max(1, (int)blockIdx.y * chunk), hi = min(m, ((int)blockIdx.y + 1) * chunk);
   for (int q = lo; q < hi; ++q) {
-    const FilterSample s = filter_sample(samples + (long long)q * 6 * ld + i, ld, mu, mu1);
-    const unsigned long long p1 = pattern(s.q1), p2 = pattern(s.q2), d = pattern(fabs(s.C - first.C));
+    const FilterSample s = filter_sample(o, samples + (long long)q * 6 * ld + i, ld, mu, mu1);
+    const unsigned long long p1 = pattern(s.q1), p2 = pattern(s.q2), d = pattern(fabs(o.sub(s.C, first.C)));
     q1 = p1 < q1 ? p1 : q1;
     q2 = p2 < q2 ? p2 : q2;
     e = d > e && d <= 0x7FF0000000000000ull ? d : e;
@@ -500,7 +506,7 @@ __global__ void filters_finish_kernel(int N, const double* samples, long long ld
                                       double* min_r2, double* max_rel_e) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const FilterSample first = filter_sample(samples + i, ld, mu, 1.0 - mu);
+  const FilterSample first = filter_sample(hg::FusedOps(), samples + i, ld, mu, 1.0 - mu);
   filter_finish(first, pattern(min_r1[i]), pattern(min_r2[i]), pattern(max_rel_e[i]), min_r1 + i, min_r2 + i,
                 max_rel_e + i);
 }
