@@ -18,7 +18,7 @@
 // bounds for the skip, the Hermite basis at the scan's points formed once per
 // warp, every point evaluated once and handed to its neighbour -- and the
 // chains of the refinements, which ran one lane at a time before they were
-// queued.  20011 trajectories x 300 segments, cubic: 4.94 -> 0.74 ms.
+// queued.  20011 trajectories x 300 segments, cubic: 4.94 -> 0.70 ms.
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -176,7 +176,11 @@ __device__ __forceinline__ bool sub_crosses(double g_lo, double g_hi, int direct
   return hg_gt0(g_lo) && (hg_lt0(g_hi) || hg_eq0(g_hi));
 }
 
-constexpr int kSecBlock = 64;
+// One warp a block: warps differ in their candidates, and a block of several
+// holds its place until the slowest is done (cubic, us, blocks of 128 / 64 / 32:
+// 500 x 301 samples 657 / 619 / 593, 20011 x 301 918 / 803 / 738, 65536 x 301
+// 1703 / 1412 / 1316).
+constexpr int kSecBlock = 32;
 constexpr int kSecQueue = 8;   // crossings a lane holds back
 constexpr int kSecBatch = 8;   // samples loaded ahead
 
