@@ -461,9 +461,7 @@ def bench_synodic_detect(args):
           {"states": n, "samples": m, "segment_refine": 50, "interp": "cubic", "max_hits": 8},
           mean_hits=hits, linear={"ms": res["linear"][0], "mean_hits": res["linear"][1]},
           roofline={"bound": "fp64", "bytes_read": sample_bytes, "achieved_gbs": sample_bytes / (ms * 1e-3) / 1e9,
-                    "fp64_pipe_active": 0.835, "dram_throughput": 0.004,
-                    "source": "ncu of section_kernel on this workload (profiles/section_kernel_synodic_65536.md): "
-                              "the cubic Hermite evaluations and refinements hold the FP64 pipe; the scanned "
+                    "source": "the cubic Hermite evaluations and refinements hold the FP64 pipe; the scanned "
                               "components are read once"})
 
 
@@ -968,7 +966,7 @@ def main():
             traffic = rec.get("dram_bytes_per_launch")
             pipe = {k: rec[k] for k in ("fp64_pipe_active", "fp64_issue_frac", "threads_per_instruction") if k in rec}
             pipe["source"] = ("from profiles/traffic_dop853_manifold.json (ncu of the dominant launch, "
-                              "profiles/dop853_manifold_16384.md), not measured in this run")
+                              "profiles/kernel_counters.md), not measured in this run")
         step_achieved = flops / (kernel_ms * 1e-3) / 1e12
         if dom is not None:
             g, dom_ms, dom_att = dom
