@@ -74,13 +74,20 @@ hg::Dir make_dir(int dim, int fwd, int flip_lo, int flip_hi) {
   return d;
 }
 
-// Allow a kernel more dynamic shared memory than a launch gets unasked.
+// Allow a kernel more dynamic shared memory than a launch gets unasked.  The
+// attribute is the kernel's, not the launch's, and host threads with a handle
+// each launch the same kernel in different shapes: so `most` is the largest
+// amount any shape of the kernel takes (a constant of the device), and no call
+// lowers what another one is about to use.
 template <class K>
-bool allow_smem(K kernel, size_t bytes) {
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess) return true;
+bool allow_smem(K kernel, size_t most) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) == cudaSuccess) return true;
   cudaGetLastError();
   return false;
 }
+
+// Shared memory that keeps a second block off an SM.
+size_t lone_block_smem(const hg_handle* h) { return (size_t)(h->smem_per_sm / 2 + 1024); }
 
 // Lanes per 6-dim trajectory when the caller did not choose.
 int auto_lanes_d6(const hg_handle* h, int N) {
@@ -96,7 +103,7 @@ int launch_fixed_d6(hg_handle* h, const hg::FixedParams& p, cudaStream_t s) {
   const int grid = (p.N + tpb - 1) / tpb;
   if (grid < 1) return HG_OK;
   const size_t smem = hg::fixed_smem_bytes<ORDER, G>(h->block);
-  if (smem > 48 * 1024 && !allow_smem(hg::fixed_rk_d6_kernel<ORDER, G>, smem))
+  if (smem > 48 * 1024 && !allow_smem(hg::fixed_rk_d6_kernel<ORDER, G>, hg::fixed_smem_bytes<ORDER, G>(128)))
     return fail(h, HG_ERR_CUDA, "shared memory");
   hg::fixed_rk_d6_kernel<ORDER, G><<<grid, h->block, smem, s>>>(p);
   return check_launch(h, "fixed_rk_d6_kernel");
@@ -167,7 +174,7 @@ int launch_dop853_pair(hg_handle* h, const hg::DopParams& p, cudaStream_t s) {
   const int grid = (p.N + per_block - 1) / per_block;
   if (grid < 1) return HG_OK;
   const size_t smem = hg::pair_dop_smem(block);
-  if (block > 64 && !allow_smem(hg::dop853_pair_kernel, smem)) return fail(h, HG_ERR_CUDA, "shared memory");
+  if (block > 64 && !allow_smem(hg::dop853_pair_kernel, hg::pair_dop_smem(128))) return fail(h, HG_ERR_CUDA, "shared memory");
   hg::dop853_pair_kernel<<<grid, block, smem, s>>>(p);
   return check_launch(h, "dop853_pair_kernel");
 }
@@ -183,9 +190,9 @@ int launch_fixed_pair(hg_handle* h, const hg::FixedParams& p, cudaStream_t s) {
   const int grid = (p.N + per_block - 1) / per_block;
   if (grid < 1) return HG_OK;
   size_t smem = hg::pair_fixed_smem<ORDER>(block);
-  const size_t half = (size_t)(h->smem_per_sm / 2 + 1024);
-  if (block == 128 && grid <= h->sm_count && half > smem) smem = half;
-  if (block > 64 && !allow_smem(hg::fixed_rk_pair_kernel<ORDER>, smem)) return fail(h, HG_ERR_CUDA, "shared memory");
+  const size_t most = std::max(hg::pair_fixed_smem<ORDER>(128), lone_block_smem(h));
+  if (block == 128 && grid <= h->sm_count) smem = most;
+  if (block > 64 && !allow_smem(hg::fixed_rk_pair_kernel<ORDER>, most)) return fail(h, HG_ERR_CUDA, "shared memory");
   hg::fixed_rk_pair_kernel<ORDER><<<grid, block, smem, s>>>(p);
   return check_launch(h, "fixed_rk_pair_kernel");
 }
@@ -340,13 +347,12 @@ struct Shape {
 template <int G, class K>
 Shape dop_shape(const hg_handle* h, K kernel) {
   Shape sh{h->block, hg::dop_smem_bytes<G>(h->block), 1};
+  const size_t most = std::max(hg::dop_smem_bytes<G>(128), lone_block_smem(h));
   if (h->spread && h->smem_per_sm > 0) {
     sh.block = 128;
-    sh.smem = std::max(hg::dop_smem_bytes<G>(128), (size_t)(h->smem_per_sm / 2 + 1024));
+    sh.smem = most;
   }
-  if (sh.smem > 32 * 1024 &&  // with the static part above the 48 KB a launch gets unasked
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem) != cudaSuccess) {
-    cudaGetLastError();
+  if (sh.smem > 32 * 1024 && !allow_smem(kernel, most)) {  // with the static part above the 48 KB a launch gets unasked
     sh.block = 32;  // fits without the attribute
     sh.smem = hg::dop_smem_bytes<G>(32);
   }
