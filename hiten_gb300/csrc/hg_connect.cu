@@ -30,6 +30,7 @@
 
 #include <algorithm>
 
+#include "hg_strided.cuh"
 #include "hitengpu.h"
 
 namespace {
@@ -310,7 +311,7 @@ __device__ __forceinline__ int cell_of(double v, double v0, double inv, int G) {
 }
 
 __global__ void grid_init_kernel(int cells, int* __restrict__ ends, GridHead* __restrict__ h) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cells; i += gridDim.x * blockDim.x) ends[i] = 0;
+  for (const int i : grid_strided(cells)) ends[i] = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     h->lo[0] = h->lo[1] = ~0ull;
     h->hi[0] = h->hi[1] = 0ull;
@@ -322,7 +323,7 @@ __global__ void grid_init_kernel(int cells, int* __restrict__ ends, GridHead* __
 __global__ void __launch_bounds__(256) grid_box_kernel(int n, const double* __restrict__ x, const double* __restrict__ y,
                                                        GridHead* __restrict__ h) {
   unsigned long long lo[2] = {~0ull, ~0ull}, hi[2] = {0, 0};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (const int i : grid_strided(n)) {
     const unsigned long long k[2] = {order_key(x[i]), order_key(y[i])};
     for (int a = 0; a < 2; ++a) {
       lo[a] = min(lo[a], k[a]);
@@ -359,7 +360,7 @@ __global__ void grid_size_kernel(int G, double reach, GridHead* __restrict__ h) 
 __global__ void grid_count_kernel(int n, const double* __restrict__ x, const double* __restrict__ y, int G,
                                   const GridHead* __restrict__ h, int* __restrict__ ends) {
   if (!h->use) return;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+  for (const int i : grid_strided(n))
     atomicAdd(&ends[cell_of(y[i], h->y0, h->inv, G) * G + cell_of(x[i], h->x0, h->inv, G)], 1);
 }
 
@@ -415,16 +416,16 @@ __global__ void __launch_bounds__(1024) grid_scan_kernel(int cells, const GridHe
 __global__ void grid_fill_kernel(int n, const double* __restrict__ x, const double* __restrict__ y, int G,
                                  const GridHead* __restrict__ h, int* __restrict__ ends, int* __restrict__ order) {
   if (!h->use) return;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+  for (const int i : grid_strided(n))
     order[atomicAdd(&ends[cell_of(y[i], h->y0, h->inv, G) * G + cell_of(x[i], h->x0, h->inv, G)], 1)] = i;
 }
 
-// Points of row cy, cells ca .. cb: order[first .. last).
+// Points of row cy, cells ca .. cb: order[first .. first + count).
 __device__ __forceinline__ void row_range(const int* __restrict__ ends, int G, int cy, int ca, int cb, int& first,
-                                          int& last) {
+                                          int& count) {
   const int c = cy * G + ca;
   first = c ? ends[c - 1] : 0;
-  last = ends[cy * G + cb];
+  count = ends[cy * G + cb] - first;
 }
 
 // Candidates the queries meet in the three by three cells around them (the
@@ -434,12 +435,12 @@ __global__ void __launch_bounds__(256) grid_work_kernel(int nq, const double* __
                                                         const int* __restrict__ ends, GridHead* __restrict__ h) {
   if (!h->use) return;
   unsigned long long work = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nq; i += gridDim.x * blockDim.x) {
+  for (const int i : grid_strided(nq)) {
     const int cx = cell_of(x[i], h->x0, h->inv, G), cy = cell_of(y[i], h->y0, h->inv, G);
     for (int r = max(cy - 1, 0); r <= min(cy + 1, G - 1); ++r) {
-      int a, b;
-      row_range(ends, G, r, max(cx - 1, 0), min(cx + 1, G - 1), a, b);
-      work += (unsigned long long)(b - a);
+      int a, c;
+      row_range(ends, G, r, max(cx - 1, 0), min(cx + 1, G - 1), a, c);
+      work += (unsigned long long)c;
     }
   }
   for (int o = 16; o; o >>= 1) work += __shfl_xor_sync(0xFFFFFFFFu, work, o);
@@ -485,7 +486,7 @@ __global__ void __launch_bounds__(128) radius_grid_kernel(int nq, const double* 
   if (!h->use) return;
   __shared__ int queue[kRadiusQueue][128];
   const int tx = threadIdx.x;
-  const int i = blockIdx.x * blockDim.x + tx;
+  const long long i = global_thread();
   const bool valid = i < nq;
   const double xi = valid ? qx[i] : 0.0, yi = valid ? qy[i] : 0.0, r2 = eps * eps;
   const float xf = near_float(xi), yf = near_float(yi), T = screen_bound(eps, R);
@@ -494,9 +495,9 @@ __global__ void __launch_bounds__(128) radius_grid_kernel(int nq, const double* 
   const int cl = cell_of(xi - reach, h->x0, h->inv, G), ch = cell_of(xi + reach, h->x0, h->inv, G);
   int row = cell_of(yi - reach, h->y0, h->inv, G);
   const int row_end = valid ? cell_of(yi + reach, h->y0, h->inv, G) : row - 1;
-  int t = 0, end = 0;
+  int t = 0, left = 0;  // next candidate of the row, candidates left in it
   bool more = valid;
-  if (valid) row_range(ends, G, row, cl, ch, t, end);
+  if (valid) row_range(ends, G, row, cl, ch, t, left);
   auto flush = [&]() {
     for (int e = 0; __any_sync(0xFFFFFFFFu, e < queued); ++e) {
       if (e >= queued) continue;
@@ -515,7 +516,7 @@ __global__ void __launch_bounds__(128) radius_grid_kernel(int nq, const double* 
     int j[4];
     double xj[4], yj[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) j[e] = t + e < end ? order[t + e] : -1;
+    for (int e = 0; e < 4; ++e) j[e] = e < left ? order[t + e] : -1;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       xj[e] = j[e] >= 0 ? rx[j[e]] : 0.0;
@@ -525,12 +526,14 @@ __global__ void __launch_bounds__(128) radius_grid_kernel(int nq, const double* 
 #pragma unroll
     for (int e = 0; e < 4; ++e)
       if (j[e] >= 0 && !(fmaxf(fabsf(xf - near_float(xj[e])), fabsf(yf - near_float(yj[e]))) > T)) queue[queued++][tx] = j[e];
-    t += 4;
-    while (more && t >= end) {
+    const int taken = min(left, 4);
+    t += taken;
+    left -= taken;
+    while (more && left == 0) {
       if (++row > row_end)
         more = false;
       else
-        row_range(ends, G, row, cl, ch, t, end);
+        row_range(ends, G, row, cl, ch, t, left);
     }
   }
   flush();
@@ -550,7 +553,7 @@ __global__ void __launch_bounds__(128) nearest_grid_kernel(int n, const double* 
                                                            const GridHead* __restrict__ h, double R,
                                                            int* __restrict__ out) {
   if (!h->use) return;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  const long long q = global_thread();
   if (q >= n) return;
   const int i = order[q];
   const double xi = x[i], yi = y[i];
@@ -570,13 +573,13 @@ __global__ void __launch_bounds__(128) nearest_grid_kernel(int n, const double* 
   float T = INFINITY;
   auto visit = [&](int r, int ca, int cb) {
     if (r < 0 || r >= G || cb < 0 || ca >= G) return;
-    int a, b;
-    row_range(ends, G, r, max(ca, 0), min(cb, G - 1), a, b);
-    for (int t = a; t < b; t += 4) {
+    int a, c;
+    row_range(ends, G, r, max(ca, 0), min(cb, G - 1), a, c);
+    for (int t = 0; t < c; t += 4) {
       int j[4];
       double xj[4], yj[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) j[e] = order[min(t + e, b - 1)];
+      for (int e = 0; e < 4; ++e) j[e] = order[a + min(t + e, c - 1)];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         xj[e] = x[j[e]];
@@ -626,14 +629,14 @@ GridHead* build_grid(int nq, const double* qx, const double* qy, int n, const do
   *ends = *order + n;
   *side = G;
   GridHead* h = (GridHead*)((char*)ws + 8 * (long long)n - 256);
-  const int blocks = (int)std::min<long long>(((long long)n + 255) / 256, 1216);
+  const unsigned blocks = std::min(blocks_of(n, 256), 1216u);
   grid_init_kernel<<<blocks, 256, 0, st>>>(cells, *ends, h);
   grid_box_kernel<<<blocks, 256, 0, st>>>(n, x, y, h);
   grid_size_kernel<<<1, 1, 0, st>>>(G, reach, h);
   grid_count_kernel<<<blocks, 256, 0, st>>>(n, x, y, G, h, *ends);
   grid_scan_kernel<<<1, 1024, 0, st>>>(cells, h, *ends);
   grid_fill_kernel<<<blocks, 256, 0, st>>>(n, x, y, G, h, *ends, *order);
-  grid_work_kernel<<<(int)std::min<long long>(((long long)nq + 255) / 256, 1216), 256, 0, st>>>(nq, qx, qy, G, *ends, h);
+  grid_work_kernel<<<std::min(blocks_of(nq, 256), 1216u), 256, 0, st>>>(nq, qx, qy, G, *ends, h);
   grid_decide_kernel<<<1, 1, 0, st>>>((unsigned long long)nq * (unsigned long long)n, h);
   return h;
 }
@@ -781,7 +784,7 @@ int hg_radius_best(int nq, const double* qx, const double* qy, int nr, const dou
     // past the rounding of the query's own coordinate and of the pair test
     const double reach = eps * (1.0 + 0x1p-40) + 0x1p-40 * coord_max;
     grid = build_grid(nq, qx, qy, nr, rx, ry, reach, rf, &ends, &order, &G, st);
-    radius_grid_kernel<<<(unsigned)((nq + 127) / 128), 128, 0, st>>>(nq, qx, qy, G, rx, ry, ends, order, grid, eps, reach,
+    radius_grid_kernel<<<blocks_of(nq, 128), 128, 0, st>>>(nq, qx, qy, G, rx, ry, ends, order, grid, eps, reach,
                                                                      coord_max, count, best_idx, best_d2);
   }
   if (nr > 0) float2_copy(nr, rx, ry, rf, grid, st);
@@ -816,7 +819,7 @@ int hg_nearest_neighbor(int n, const double* x, const double* y, double coord_ma
   if (grid_worth(n, n)) {
     int *ends, *order, G;
     grid = build_grid(n, x, y, n, x, y, 0.0, pf, &ends, &order, &G, st);
-    nearest_grid_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(n, x, y, G, ends, order, grid, coord_max, out);
+    nearest_grid_kernel<<<blocks_of(n, 128), 128, 0, st>>>(n, x, y, G, ends, order, grid, coord_max, out);
   }
   float2_copy(n, x, y, pf, grid, st);
   const int S = lanes_per_query(nearest_kernel<8>, n);
