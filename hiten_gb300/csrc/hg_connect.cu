@@ -25,8 +25,9 @@
 // count on the device.  65536 x 65536 points on two noisy curves: radius 1.47 ->
 // 0.20 ms, nearest 2.74 -> 0.26 ms with the grid (0.05 ms).
 #include <cuda_runtime.h>
-#include <stdint.h>
+#include <limits.h>
 #include <math.h>
+#include <stdint.h>
 
 #include <algorithm>
 
@@ -65,11 +66,12 @@ struct GridHead {
   unsigned long long work;          // candidates of all queries
   double x0, y0, inv, cell;         // cell of x: floor((x - x0) inv)
   int use;                          // search through the grid
+  int far;                          // it left queries to nearest_far_kernel
 };
 
 __global__ void to_float2_kernel(int n, const double* __restrict__ x, const double* __restrict__ y,
                                  float2* __restrict__ out, const GridHead* __restrict__ grid) {
-  if (grid && grid->use) return;
+  if (grid && grid->use && !grid->far) return;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     out[i] = make_float2((float)x[i], (float)y[i]);
 }
@@ -317,6 +319,7 @@ __global__ void grid_init_kernel(int cells, int* __restrict__ ends, GridHead* __
     h->hi[0] = h->hi[1] = 0ull;
     h->work = 0;
     h->use = 0;
+    h->far = 0;
   }
 }
 
@@ -543,39 +546,120 @@ __global__ void __launch_bounds__(128) radius_grid_kernel(int nq, const double* 
   best_d2[i] = bj < 0 ? 0.0 : bd;
 }
 
+// The nearest point a query has met: the smallest squared distance below the
+// all-pairs scan's first acceptance, ties to the smaller index.  FP32 distances
+// decide while they can: a point is passed over when another one is certainly
+// nearer, takes the place of one that is certainly farther, and only what lies in
+// between is decided in FP64 (a search whose every improvement was, ln(c) a lane
+// of c candidates, held the FP64 unit).
+//
+// With coordinates within 2^-23 R a distance f is off by at most a(f) = 2^-21.8 f
+// + 2^-20.4 R sqrt(f) + 2^-43 R^2 (the header's derivation).  A point at g >
+// f + E(f), E(f) = 2^-20 f + 2^-19 R sqrt(f) + 2^-38 R^2, is farther than one at f:
+// g - a(g) grows from 2^-42.8 R^2 on, and at g = f + E(f) it exceeds f + a(f),
+// as a(f) + a(f + E(f)) < E(f) (sqrt(f + E) <= sqrt(f) + sqrt(E)).  2^-120 more
+// for squares below FP32's range; beyond it (R^2 infinite) E is infinite and every
+// point is decided in FP64.
+struct Nearest {
+  double x, y;
+  float xf, yf, R2, RR;
+  float least, cut;  // FP32 distance of `at`; beyond `cut` a point is farther
+  int at;            // nearest so far, not decided (-1: none)
+  double bd;         // decided
+  int bj;
+  __device__ __forceinline__ Nearest(double px, double py, double R)
+      : x(px), y(py), xf(near_float(px)), yf(near_float(py)), least(INFINITY), cut(INFINITY), at(-1), bd(1e300), bj(-1) {
+    const float Rf = __double2float_ru(R);
+    R2 = 2.0f * Rf;
+    RR = fmaf(0x1p-38f * Rf, Rf, 0x1p-120f);
+  }
+  __device__ __forceinline__ float beyond(float d2) const {
+    float s;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(s) : "f"(d2));
+    return fmaf(0x1p-20f, fmaf(R2, s, d2), RR) + d2;
+  }
+  __device__ __forceinline__ void decide(double xj, double yj, int j) {
+    const double dx = x - xj, dy = y - yj;
+    const double d2 = dx * dx + dy * dy;
+    if (d2 < bd || (d2 == bd && bj >= 0 && j < bj)) {
+      bd = d2;
+      bj = j;
+    }
+  }
+  // a point decided elsewhere
+  __device__ __forceinline__ void take(double d2, int j) {
+    if (d2 < bd || (d2 == bd && (unsigned)j < (unsigned)bj)) {
+      bd = d2;
+      bj = j;
+    }
+  }
+  __device__ __forceinline__ void settle(const double* px, const double* py) {
+    if (at >= 0) decide(px[at], py[at], at);
+    at = -1;
+  }
+  __device__ __forceinline__ float distance(float fx, float fy) const {
+    const float dx = xf - fx, dy = yf - fy;
+    return fmaf(dx, dx, dy * dy);
+  }
+  __device__ __forceinline__ void meet(double xj, double yj, int j, const double* px, const double* py) {
+    const float d2 = distance(near_float(xj), near_float(yj));
+    if (d2 > cut) return;
+    const float c = d2 < least ? beyond(d2) : INFINITY;
+    if (c < least) {  // nearer than any so far
+      at = j;
+      bd = 1e300;
+      bj = -1;
+    } else {
+      settle(px, py);
+      decide(xj, yj, j);
+    }
+    least = fminf(least, d2);
+    cut = fminf(cut, c);
+  }
+};
+
 // Nearest neighbours: a query (in cell order, so that a warp's meet the same
 // cells) takes the three by three cells around its own, then ring after ring
-// until the block's border is farther than the best found.
+// until the block's border is farther than the best found.  A query whose
+// nearest point lies beyond kRings rings, or whose rings meet more than a 64th
+// of all points, is left to nearest_far_kernel (kFar in `out`): its walk, two
+// dependent loads a row and side and two for every four candidates, would go on
+// alone, for up to G rings.
+//
+// S lanes share a query: the cells' candidates, or a ring's rows and sides.  The
+// loads' latency bounds it, and far points make it longer: they widen the box and
+// with it the cells (434 candidates a query of 65536 points on a noisy curve, 1432
+// with a hundred points strewn around it).  Against one lane a query, every ring
+// walked to its end and every improvement decided in FP64, ms: the curve 0.28 ->
+// 0.18, with one far point 7.17 -> 0.28, with a hundred 2.13 -> 0.60; 16384 points
+// 0.14 -> 0.08, 1.90 -> 0.11, 0.47 -> 0.19.
+constexpr int kRings = 4;
+constexpr int kFar = -2;
+template <int S>
 __global__ void __launch_bounds__(128) nearest_grid_kernel(int n, const double* __restrict__ x,
                                                            const double* __restrict__ y, int G,
                                                            const int* __restrict__ ends,
                                                            const int* __restrict__ order,
-                                                           const GridHead* __restrict__ h, double R,
+                                                           GridHead* __restrict__ h, double R,
                                                            int* __restrict__ out) {
   if (!h->use) return;
-  const long long q = global_thread();
+  const long long q = global_thread() / S;
   if (q >= n) return;
+  const int s = threadIdx.x % S;
+  const unsigned group = ((1u << S) - 1u) << ((threadIdx.x & 31) - s);
   const int i = order[q];
-  const double xi = x[i], yi = y[i];
-  const float xf = near_float(xi), yf = near_float(yi);
-  // screen_bound(sqrt(bd), R) in FP32: the root's argument (truncated) and the
-  // root up by 2^-15 each, 2^-62 for a distance below FP32's range
-  const float R21 = screen_bound(0.0, R);
-  auto bound = [&](double d2) {
-    float s;
-    asm("sqrt.approx.f32 %0, %1;" : "=f"(s) : "f"(near_float(d2) * 1.0001f));
-    return fmaf(s, 1.0001f, R21) + 0x1p-62f;
-  };
+  Nearest best(x[i], y[i], R);
   const double x0 = h->x0, y0 = h->y0, cell = h->cell;
-  const int cx = cell_of(xi, x0, h->inv, G), cy = cell_of(yi, y0, h->inv, G);
-  int bj = -1;
-  double bd = 1e300;  // the all-pairs scan's first acceptance
-  float T = INFINITY;
-  auto visit = [&](int r, int ca, int cb) {
-    if (r < 0 || r >= G || cb < 0 || ca >= G) return;
+  const int cx = cell_of(best.x, x0, h->inv, G), cy = cell_of(best.y, y0, h->inv, G);
+  int budget = INT_MAX;  // candidates this lane may still meet; below zero: too many
+  // row r's cells ca .. cb; `part` of the row's `parts` lanes
+  auto visit = [&](int r, int ca, int cb, int part, int parts) {
+    if (r < 0 || r >= G || cb < 0 || ca >= G || budget < 0) return;
     int a, c;
     row_range(ends, G, r, max(ca, 0), min(cb, G - 1), a, c);
-    for (int t = 0; t < c; t += 4) {
+    budget = c > budget ? -1 : budget - c;
+    if (budget < 0) return;
+    for (int t = 4 * part; t < c; t += 4 * parts) {
       int j[4];
       double xj[4], yj[4];
 #pragma unroll
@@ -586,38 +670,136 @@ __global__ void __launch_bounds__(128) nearest_grid_kernel(int n, const double* 
         yj[e] = y[j[e]];
       }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {  // (a repeated last candidate changes nothing)
-        if (fmaxf(fabsf(xf - near_float(xj[e])), fabsf(yf - near_float(yj[e]))) > T || j[e] == i) continue;
-        const double dx = xi - xj[e], dy = yi - yj[e];
-        const double d2 = dx * dx + dy * dy;
-        if (d2 < bd || (d2 == bd && bj >= 0 && j[e] < bj)) {
-          bd = d2;
-          bj = j[e];
-          T = bound(d2);
-        }
-      }
+      for (int e = 0; e < 4; ++e)  // (a repeated last candidate changes nothing)
+        if (j[e] != i) best.meet(xj[e], yj[e], j[e], x, y);
     }
   };
-  for (int r = cy - 1; r <= cy + 1; ++r) visit(r, cx - 1, cx + 1);
+  // what the lanes found, in each of them
+  auto share = [&]() {
+    best.settle(x, y);
+    for (int o = 1; o < S; o <<= 1) {
+      const double d2 = __shfl_xor_sync(group, best.bd, o);
+      const int j = __shfl_xor_sync(group, best.bj, o);
+      best.least = fminf(best.least, __shfl_xor_sync(group, best.least, o));
+      best.cut = fminf(best.cut, __shfl_xor_sync(group, best.cut, o));
+      budget = min(budget, __shfl_xor_sync(group, budget, o));
+      best.take(d2, j);
+    }
+  };
+  // (its own row first: what it finds there rules out most of the others')
+  visit(cy, cx - 1, cx + 1, s, S);
+  visit(cy - 1, cx - 1, cx + 1, s, S);
+  visit(cy + 1, cx - 1, cx + 1, s, S);
+  budget = n / 64;
   for (int k = 1;; ++k) {
+    share();
     // every point outside the block of radius k is at least this far away (the
     // cells' borders are off by their rounding)
     double far = INFINITY;
-    if (cx - k > 0) far = fmin(far, xi - (x0 + (double)(cx - k) * cell));
-    if (cx + k + 1 < G) far = fmin(far, (x0 + (double)(cx + k + 1) * cell) - xi);
-    if (cy - k > 0) far = fmin(far, yi - (y0 + (double)(cy - k) * cell));
-    if (cy + k + 1 < G) far = fmin(far, (y0 + (double)(cy + k + 1) * cell) - yi);
-    if (!(far < INFINITY)) break;  // the block covers the grid
-    far = far * (1.0 - 0x1p-40) - 0x1p-40 * (R + cell);
-    if (far > 0.0 && far * far * (1.0 - 0x1p-40) > bd) break;
-    visit(cy - k - 1, cx - k - 1, cx + k + 1);
-    visit(cy + k + 1, cx - k - 1, cx + k + 1);
-    for (int r = cy - k; r <= cy + k; ++r) {
-      visit(r, cx - k - 1, cx - k - 1);
-      visit(r, cx + k + 1, cx + k + 1);
+    if (cx - k > 0) far = fmin(far, best.x - (x0 + (double)(cx - k) * cell));
+    if (cx + k + 1 < G) far = fmin(far, (x0 + (double)(cx + k + 1) * cell) - best.x);
+    if (cy - k > 0) far = fmin(far, best.y - (y0 + (double)(cy - k) * cell));
+    if (cy + k + 1 < G) far = fmin(far, (y0 + (double)(cy + k + 1) * cell) - best.y);
+    if (budget >= 0) {
+      if (!(far < INFINITY)) break;  // the block covers the grid
+      far = far * (1.0 - 0x1p-40) - 0x1p-40 * (R + cell);
+      if (far > 0.0 && far * far * (1.0 - 0x1p-40) > best.bd) break;
+    }
+    if (k > kRings || budget < 0) {
+      best.bj = kFar;
+      h->far = 1;
+      break;
+    }
+    // the ring: two rows, then 2 k + 1 cells of each side
+    for (int u = s; u < 4 * k + 4; u += S) {
+      const int v = u - 2, side = (v & 1) ? cx + k + 1 : cx - k - 1;
+      if (v < 0)
+        visit(u == 0 ? cy - k - 1 : cy + k + 1, cx - k - 1, cx + k + 1, 0, 1);
+      else
+        visit(cy - k + (v >> 1), side, side, 0, 1);
     }
   }
-  out[i] = bj;
+  if (s == 0) out[i] = best.bj;
+}
+
+// The queries nearest_grid_kernel left, a block each, over all points.  Either
+// they lie five cells from any other point, so with no more cells than points
+// there are at most about n / 16 of them; or a cell or more from any other, within
+// five of a 64th of all points, which leaves room for a few thousand.  A block's
+// share is strided: far points tend to follow each other.  Two passes, as the
+// all-pairs scan: the block's least FP32 distance, then what it does not rule out.
+constexpr int kFarBlock = 512, kFarTile = 8 * kFarBlock;
+__global__ void __launch_bounds__(kFarBlock) nearest_far_kernel(int n, const double* __restrict__ x,
+                                                                const double* __restrict__ y,
+                                                                const float2* __restrict__ pf,
+                                                                const GridHead* __restrict__ h, double R,
+                                                                int* __restrict__ out) {
+  if (!h->use || !h->far) return;
+  __shared__ int list[kFarBlock], listed;
+  __shared__ double warp_d[kFarBlock / 32];
+  __shared__ int warp_j[kFarBlock / 32];
+  __shared__ float warp_least[kFarBlock / 32];
+  const int tx = threadIdx.x;
+  const unsigned keep = n - kHeadPoints, tiles = keep / kFarTile;
+  for (long long base = 0; blockIdx.x + base * gridDim.x < n; base += kFarBlock) {
+    const long long q = blockIdx.x + (base + tx) * gridDim.x;
+    const bool far = q < n && out[q] == kFar;
+    if (tx == 0) listed = 0;
+    if (!__syncthreads_or(far)) continue;
+    if (far) list[atomicAdd(&listed, 1)] = (int)q;
+    __syncthreads();
+    const int m = listed;
+    for (int u = 0; u < m; ++u) {
+      const int i = list[u];
+      Nearest best(x[i], y[i], R);
+      // FP32 distances of this thread's points (as many iterations in every thread)
+      auto scan = [&](auto meet) {
+        unsigned b = tx;
+        for (unsigned t = 0; t < tiles; ++t, b += kFarTile) {
+          float2 f[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) f[e] = pf[b + e * kFarBlock];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) meet(best.distance(f[e].x, f[e].y), b + e * kFarBlock);
+        }
+        for (; b < (unsigned)n; b += kFarBlock) {
+          const float2 f = b < keep ? pf[b] : make_float2((float)x[b], (float)y[b]);
+          meet(best.distance(f.x, f.y), b);
+        }
+      };
+      float least = INFINITY;
+      scan([&](float d2, unsigned j) { least = fminf(least, j == (unsigned)i ? INFINITY : d2); });
+      least = __uint_as_float(__reduce_min_sync(0xFFFFFFFFu, __float_as_uint(least)));
+      if ((tx & 31) == 0) warp_least[tx >> 5] = least;
+      __syncthreads();
+      least = __uint_as_float(
+          __reduce_min_sync(0xFFFFFFFFu, __float_as_uint(warp_least[(tx & 31) % (kFarBlock / 32)])));
+      const float cut = best.beyond(least);
+      scan([&](float d2, unsigned j) {
+        if (!(d2 > cut) && j != (unsigned)i) best.decide(x[j], y[j], (int)j);
+      });
+      auto over_warp = [&]() {
+        for (int o = 16; o; o >>= 1) {
+          const double d2 = __shfl_xor_sync(0xFFFFFFFFu, best.bd, o);
+          const int j = __shfl_xor_sync(0xFFFFFFFFu, best.bj, o);
+          best.take(d2, j);
+        }
+      };
+      over_warp();
+      if ((tx & 31) == 0) {
+        warp_d[tx >> 5] = best.bd;
+        warp_j[tx >> 5] = best.bj;
+      }
+      __syncthreads();
+      if (tx < 32) {
+        best.bd = warp_d[tx % (kFarBlock / 32)];
+        best.bj = warp_j[tx % (kFarBlock / 32)];
+        over_warp();
+        if (tx == 0) out[i] = best.bj;
+      }
+      __syncthreads();
+    }
+  }
 }
 
 // Builds the grid of n reference points in ws and decides whether the nq
@@ -642,17 +824,17 @@ GridHead* build_grid(int nq, const double* qx, const double* qy, int n, const do
 }
 bool grid_worth(long long nq, long long n) { return n >= kGridMin && nq * n > kGridPairs; }
 
-// Lanes per query: the largest of 8, 4, 2, 1 whose grid still fits in one
-// wave of resident blocks (more lanes per query shorten each lane's scan;
+// Lanes per query: the largest of `most`, most / 2, ... 1 whose grid still fits in
+// one wave of resident blocks (more lanes per query shorten each lane's scan;
 // a second partial wave would cost a whole extra scan).
 template <class K>
-int lanes_per_query(K k8, long long n) {
+int lanes_per_query(K kernel, long long n, int block = kBlock, int most = 8) {
   int dev = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k8, kBlock, 0) != cudaSuccess)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0) != cudaSuccess)
     return 1;
-  const long long resident = (long long)sms * per_sm * kBlock;
-  for (int S = 8; S > 1; S >>= 1)
+  const long long resident = (long long)sms * per_sm * block;
+  for (int S = most; S > 1; S >>= 1)
     if (n * S <= resident) return S;
   return 1;
 }
@@ -753,7 +935,7 @@ void* points_ws(int n, void* ws, long long ws_bytes, bool* owned, cudaStream_t s
 }
 
 // FP32 copy of a point set in its workspace (left out where the grid, whose
-// storage it takes, is used).
+// storage it takes, answered every query).
 void float2_copy(int n, const double* x, const double* y, float2* out, const GridHead* grid, cudaStream_t st) {
   const int blocks = (int)std::min<long long>(((long long)n + 255) / 256, 4096);
   to_float2_kernel<<<blocks, 256, 0, st>>>(grid ? n - kHeadPoints : n, x, y, out, grid);
@@ -819,9 +1001,17 @@ int hg_nearest_neighbor(int n, const double* x, const double* y, double coord_ma
   if (grid_worth(n, n)) {
     int *ends, *order, G;
     grid = build_grid(n, x, y, n, x, y, 0.0, pf, &ends, &order, &G, st);
-    nearest_grid_kernel<<<blocks_of(n, 128), 128, 0, st>>>(n, x, y, G, ends, order, grid, coord_max, out);
+    const int S = lanes_per_query(nearest_grid_kernel<4>, n, 128, 4);
+    const unsigned blocks = blocks_of((long long)n * S, 128);
+    if (S == 4)
+      nearest_grid_kernel<4><<<blocks, 128, 0, st>>>(n, x, y, G, ends, order, grid, coord_max, out);
+    else if (S == 2)
+      nearest_grid_kernel<2><<<blocks, 128, 0, st>>>(n, x, y, G, ends, order, grid, coord_max, out);
+    else
+      nearest_grid_kernel<1><<<blocks, 128, 0, st>>>(n, x, y, G, ends, order, grid, coord_max, out);
   }
   float2_copy(n, x, y, pf, grid, st);
+  if (grid) nearest_far_kernel<<<304, kFarBlock, 0, st>>>(n, x, y, pf, grid, coord_max, out);
   const int S = lanes_per_query(nearest_kernel<8>, n);
   const long long blocks = ((long long)n * S + kBlock - 1) / kBlock;
   if (S == 8)
