@@ -48,30 +48,32 @@ struct Tile {
   float2 f[kTile];
 };
 
-// FP32 copy of points [0, keep) (pf), converted here beyond.
-__device__ __forceinline__ void load_tile(Tile& T, const float2* __restrict__ pf, const double* __restrict__ x,
-                                          const double* __restrict__ y, int keep, int base, int n) {
-  for (int t = threadIdx.x; t < n; t += blockDim.x) {
-    const int j = base + t;
-    T.f[t] = j < keep ? pf[j] : make_float2((float)x[j], (float)y[j]);
-  }
+__device__ __forceinline__ void load_tile(Tile& T, const float2* __restrict__ pf, int base, int n) {
+  for (int t = threadIdx.x; t < n; t += blockDim.x) T.f[t] = pf[base + t];
 }
 
-// The grid's numbers, in the last 256 bytes of the workspace's 8 n; the FP32
-// copy leaves them alone (kHeadPoints points are converted where they are
-// used).
+// The grid's numbers, in the last 256 bytes of the workspace's 8 n.  Where the
+// grid is not used the FP32 copy takes their place too (the all-pairs scans have
+// no registers to spare for points that it leaves out), so `use` is set by a
+// pattern no FP32 copy has: two NaNs that no conversion returns.
 constexpr int kHeadPoints = 32;
+constexpr unsigned long long kUse = 0x7FA5A5A57FA5A5A5ull;
 struct GridHead {
   unsigned long long lo[2], hi[2];  // bounding box as ordered keys
   unsigned long long work;          // candidates of all queries
   double x0, y0, inv, cell;         // cell of x: floor((x - x0) inv)
-  int use;                          // search through the grid
+  unsigned long long use;           // kUse: search through the grid
   int far;                          // it left queries to nearest_far_kernel
+  __device__ __forceinline__ bool used() const { return use == kUse; }
 };
+static_assert(sizeof(GridHead) <= 8 * kHeadPoints, "");
 
 __global__ void to_float2_kernel(int n, const double* __restrict__ x, const double* __restrict__ y,
                                  float2* __restrict__ out, const GridHead* __restrict__ grid) {
-  if (grid && grid->use && !grid->far) return;
+  if (grid && grid->used()) {
+    if (!grid->far) return;
+    n -= kHeadPoints;
+  }
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     out[i] = make_float2((float)x[i], (float)y[i]);
 }
@@ -133,10 +135,9 @@ __global__ void __launch_bounds__(kBlock, 16) radius_best_kernel(int nq, const d
                                                               int* __restrict__ count, int* __restrict__ best_idx,
                                                               double* __restrict__ best_d2,
                                                               const GridHead* __restrict__ grid) {
-  if (grid && grid->use) return;  // searched through the grid
+  if (grid && grid->used()) return;  // searched through the grid
   __shared__ Tile tile;
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int keep = grid ? nr - kHeadPoints : nr;
   const int s = (int)(g % S);
   const long long i = g / S;
   const bool active = i < nq;
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(kBlock, 16) radius_best_kernel(int nq, const d
   for (int base = 0; base < nr; base += kTile) {
     const int n = min(kTile, nr - base);
     __syncthreads();
-    load_tile(tile, rf, rx, ry, keep, base, n);
+    load_tile(tile, rf, base, n);
     __syncthreads();
     if (active) {
       if (n == kTile)
@@ -235,10 +236,9 @@ __global__ void __launch_bounds__(kBlock, 16) nearest_kernel(int n, const double
                                                               const float2* __restrict__ pf, double R, double R2c,
                                                               int* __restrict__ out,
                                                               const GridHead* __restrict__ grid) {
-  if (grid && grid->use) return;  // searched through the grid
+  if (grid && grid->used()) return;  // searched through the grid
   __shared__ Tile tile;
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int keep = grid ? n - kHeadPoints : n;
   const int s = (int)(g % S);
   const long long i = g / S;
   const bool active = i < n;
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(kBlock, 16) nearest_kernel(int n, const double
   for (int base = 0; base < n; base += kTile) {
     const int cnt = min(kTile, n - base);
     __syncthreads();
-    load_tile(tile, pf, px, py, keep, base, cnt);
+    load_tile(tile, pf, base, cnt);
     __syncthreads();
     if (active) {
       const long long self = i - base;
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kBlock, 16) nearest_kernel(int n, const double
   for (int base = 0; base < n; base += kTile) {
     const int cnt = min(kTile, n - base);
     __syncthreads();
-    load_tile(tile, pf, px, py, keep, base, cnt);
+    load_tile(tile, pf, base, cnt);
     __syncthreads();
     if (active) {
       const long long self = i - base;
@@ -290,7 +290,14 @@ __global__ void __launch_bounds__(kBlock, 16) nearest_kernel(int n, const double
 // coordinate is a monotone function of it (every rounding is), so all points
 // with x in [a, b] lie in the cells cell(a) .. cell(b).
 // ---------------------------------------------------------------------------
-constexpr long long kGridPairs = 1ll << 26;  // below, the all-pairs scan takes as long as building the grid (25 us)
+// Pairs above which the grid is built.  Building it takes 40 us, which a set that
+// turns out too crowded for it pays beside the all-pairs scan (nearest: 8300
+// points 260 -> 299 us, 24000 1397 -> 1436).  All pairs / grid, us, on a noisy
+// curve and with a hundred points strewn around it:
+//                8300               12000              16384
+//   nearest   114 / 70, 115 / 122   177 / 78, 177 / 148   230 / 81, 229 / 193
+//   radius     62 / 64,  60 / 77     87 / 68,  85 / 87    117 / 72, 119 / 95
+constexpr long long kNearestPairs = 1ll << 26, kRadiusPairs = 1ll << 27;
 constexpr int kGridMin = 4096;
 
 __host__ __device__ inline int grid_side(int n) {
@@ -357,21 +364,67 @@ __global__ void grid_size_kernel(int G, double reach, GridHead* __restrict__ h) 
   h->y0 = fine ? y0 : 0.0;
   h->cell = fine ? cell : 1.0;
   h->inv = fine ? 1.0 / cell : 0.0;
-  h->use = fine ? 1 : 0;
+  h->use = fine ? kUse : 0;
+}
+
+// Adds a warp's 32 points (cell -1: none) to their cells' numbers, one atomic a
+// cell, and returns each point's own number: crowded points would otherwise
+// queue one by one at their cell's address (65536 of them, twice: 0.9 ms).
+__device__ __forceinline__ int add_to_cell(int* __restrict__ cells, int cell) {
+  const int lane = threadIdx.x & 31;
+  const unsigned same = __match_any_sync(0xFFFFFFFFu, cell);
+  const int first = __ffs(same) - 1;
+  int at = 0;
+  if (lane == first && cell >= 0) at = atomicAdd(&cells[cell], __popc(same));
+  return __shfl_sync(0xFFFFFFFFu, at, first) + __popc(same & ((1u << lane) - 1u));
+}
+
+// Calls f(i, cell) for every point, a warp's lanes together (i = n, cell -1 beyond).
+template <class F>
+__device__ __forceinline__ void each_cell(int n, const double* __restrict__ x, const double* __restrict__ y, int G,
+                                          const GridHead* __restrict__ h, F f) {
+  const int lane = threadIdx.x & 31;
+  for (const int b : Strided{global_thread() - lane, (long long)gridDim.x * blockDim.x, n}) {
+    const bool in = lane < n - b;
+    const int i = in ? b + lane : n;
+    f(i, in ? cell_of(y[i], h->y0, h->inv, G) * G + cell_of(x[i], h->x0, h->inv, G) : -1);
+  }
 }
 
 __global__ void grid_count_kernel(int n, const double* __restrict__ x, const double* __restrict__ y, int G,
-                                  const GridHead* __restrict__ h, int* __restrict__ ends) {
-  if (!h->use) return;
-  for (const int i : grid_strided(n))
-    atomicAdd(&ends[cell_of(y[i], h->y0, h->inv, G) * G + cell_of(x[i], h->x0, h->inv, G)], 1);
+                                  const GridHead* __restrict__ h, int* __restrict__ counts) {
+  if (!h->used()) return;
+  each_cell(n, x, y, G, h, [&](int, int cell) { add_to_cell(counts, cell); });
+}
+
+// Candidates the queries meet in the three by three cells around them (the
+// radius search's; nearly the nearest search's), from the cells' counts: a grid
+// that is not worth using is neither scanned nor filled.
+__global__ void __launch_bounds__(256) grid_work_kernel(int nq, const double* __restrict__ x,
+                                                        const double* __restrict__ y, int G,
+                                                        const int* __restrict__ counts, GridHead* __restrict__ h) {
+  if (!h->used()) return;
+  unsigned long long work = 0;
+  for (const int i : grid_strided(nq)) {
+    const int cx = cell_of(x[i], h->x0, h->inv, G), cy = cell_of(y[i], h->y0, h->inv, G);
+    for (int r = max(cy - 1, 0); r <= min(cy + 1, G - 1); ++r)
+      for (int c = max(cx - 1, 0); c <= min(cx + 1, G - 1); ++c) work += (unsigned)counts[r * G + c];
+  }
+  for (int o = 16; o; o >>= 1) work += __shfl_xor_sync(0xFFFFFFFFu, work, o);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&h->work, work);
 }
 
 // Counts to starts (one block; 16384 cells' loads in flight at once, scanned
-// 4096 at a time).
-__global__ void __launch_bounds__(1024) grid_scan_kernel(int cells, const GridHead* __restrict__ h,
+// 4096 at a time), if the grid pays: while it meets at most a sixteenth of the
+// pairs (a candidate costs several pairs of the all-pairs scan: two dependent
+// loads).
+__global__ void __launch_bounds__(1024) grid_scan_kernel(int cells, unsigned long long pairs, GridHead* __restrict__ h,
                                                          int* __restrict__ ends) {
-  if (!h->use) return;
+  if (!h->used()) return;
+  if (h->work > pairs / 16) {
+    if (threadIdx.x == 0) h->use = 0;
+    return;
+  }
   constexpr int kRounds = 4;
   __shared__ int warp_sum[2][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -418,9 +471,11 @@ __global__ void __launch_bounds__(1024) grid_scan_kernel(int cells, const GridHe
 // Points into their cells; the starts become the ends.
 __global__ void grid_fill_kernel(int n, const double* __restrict__ x, const double* __restrict__ y, int G,
                                  const GridHead* __restrict__ h, int* __restrict__ ends, int* __restrict__ order) {
-  if (!h->use) return;
-  for (const int i : grid_strided(n))
-    order[atomicAdd(&ends[cell_of(y[i], h->y0, h->inv, G) * G + cell_of(x[i], h->x0, h->inv, G)], 1)] = i;
+  if (!h->used()) return;
+  each_cell(n, x, y, G, h, [&](int i, int cell) {
+    const int at = add_to_cell(ends, cell);
+    if (cell >= 0) order[at] = i;
+  });
 }
 
 // Points of row cy, cells ca .. cb: order[first .. first + count).
@@ -429,31 +484,6 @@ __device__ __forceinline__ void row_range(const int* __restrict__ ends, int G, i
   const int c = cy * G + ca;
   first = c ? ends[c - 1] : 0;
   count = ends[cy * G + cb] - first;
-}
-
-// Candidates the queries meet in the three by three cells around them (the
-// radius search's; nearly the nearest search's).
-__global__ void __launch_bounds__(256) grid_work_kernel(int nq, const double* __restrict__ x,
-                                                        const double* __restrict__ y, int G,
-                                                        const int* __restrict__ ends, GridHead* __restrict__ h) {
-  if (!h->use) return;
-  unsigned long long work = 0;
-  for (const int i : grid_strided(nq)) {
-    const int cx = cell_of(x[i], h->x0, h->inv, G), cy = cell_of(y[i], h->y0, h->inv, G);
-    for (int r = max(cy - 1, 0); r <= min(cy + 1, G - 1); ++r) {
-      int a, c;
-      row_range(ends, G, r, max(cx - 1, 0), min(cx + 1, G - 1), a, c);
-      work += (unsigned long long)c;
-    }
-  }
-  for (int o = 16; o; o >>= 1) work += __shfl_xor_sync(0xFFFFFFFFu, work, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(&h->work, work);
-}
-
-// The grid pays while it meets at most a sixteenth of the pairs (a candidate
-// costs several pairs of the all-pairs scan: two dependent loads).
-__global__ void grid_decide_kernel(unsigned long long pairs, GridHead* __restrict__ h) {
-  if (h->work > pairs / 16) h->use = 0;
 }
 
 // An FP32 value within 2^-23 |v| of v, 2^-126 where v is smaller than that, and
@@ -477,7 +507,10 @@ __device__ __forceinline__ float screen_bound(double reach, double R) {
 // A warp's queries scan side by side; what passes the FP32 screen waits in a
 // queue per lane, so that the FP64 decisions run on all lanes at once instead of
 // whenever one of them has a pair.
+// S lanes share a query's candidates (one / four lanes, us: 16384 points on a curve
+// 103 / 72, with a hundred points around it 177 / 96).
 constexpr int kRadiusQueue = 8;
+template <int S>
 __global__ void __launch_bounds__(128) radius_grid_kernel(int nq, const double* __restrict__ qx,
                                                           const double* __restrict__ qy, int G,
                                                           const double* __restrict__ rx,
@@ -486,10 +519,11 @@ __global__ void __launch_bounds__(128) radius_grid_kernel(int nq, const double* 
                                                           const GridHead* __restrict__ h, double eps, double reach,
                                                           double R, int* __restrict__ count,
                                                           int* __restrict__ best_idx, double* __restrict__ best_d2) {
-  if (!h->use) return;
+  if (!h->used()) return;
   __shared__ int queue[kRadiusQueue][128];
   const int tx = threadIdx.x;
-  const long long i = global_thread();
+  const long long i = global_thread() / S;
+  const int s = tx % S;
   const bool valid = i < nq;
   const double xi = valid ? qx[i] : 0.0, yi = valid ? qy[i] : 0.0, r2 = eps * eps;
   const float xf = near_float(xi), yf = near_float(yi), T = screen_bound(eps, R);
@@ -498,9 +532,18 @@ __global__ void __launch_bounds__(128) radius_grid_kernel(int nq, const double* 
   const int cl = cell_of(xi - reach, h->x0, h->inv, G), ch = cell_of(xi + reach, h->x0, h->inv, G);
   int row = cell_of(yi - reach, h->y0, h->inv, G);
   const int row_end = valid ? cell_of(yi + reach, h->y0, h->inv, G) : row - 1;
-  int t = 0, left = 0;  // next candidate of the row, candidates left in it
+  int t = 0, left = 0;  // this lane's next candidate of the row, the row's from there on
   bool more = valid;
-  if (valid) row_range(ends, G, row, cl, ch, t, left);
+  auto skip = [&](int by) {
+    const int taken = min(left, by);
+    t += taken;
+    left -= taken;
+  };
+  auto next_row = [&]() {
+    row_range(ends, G, row, cl, ch, t, left);
+    skip(4 * s);
+  };
+  if (valid) next_row();
   auto flush = [&]() {
     for (int e = 0; __any_sync(0xFFFFFFFFu, e < queued); ++e) {
       if (e >= queued) continue;
@@ -529,18 +572,22 @@ __global__ void __launch_bounds__(128) radius_grid_kernel(int nq, const double* 
 #pragma unroll
     for (int e = 0; e < 4; ++e)
       if (j[e] >= 0 && !(fmaxf(fabsf(xf - near_float(xj[e])), fabsf(yf - near_float(yj[e]))) > T)) queue[queued++][tx] = j[e];
-    const int taken = min(left, 4);
-    t += taken;
-    left -= taken;
+    skip(4 * S);
     while (more && left == 0) {
       if (++row > row_end)
         more = false;
       else
-        row_range(ends, G, row, cl, ch, t, left);
+        next_row();
     }
   }
   flush();
-  if (!valid) return;
+  for (int o = 1; o < S; o <<= 1) {
+    c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
+    const double d2 = __shfl_xor_sync(0xFFFFFFFFu, bd, o);
+    const int j = __shfl_xor_sync(0xFFFFFFFFu, bj, o);
+    take_best(bd, bj, d2, j);
+  }
+  if (!valid || s != 0) return;
   count[i] = c;
   best_idx[i] = bj;
   best_d2[i] = bj < 0 ? 0.0 : bd;
@@ -642,7 +689,7 @@ __global__ void __launch_bounds__(128) nearest_grid_kernel(int n, const double* 
                                                            const int* __restrict__ order,
                                                            GridHead* __restrict__ h, double R,
                                                            int* __restrict__ out) {
-  if (!h->use) return;
+  if (!h->used()) return;
   const long long q = global_thread() / S;
   if (q >= n) return;
   const int s = threadIdx.x % S;
@@ -734,7 +781,7 @@ __global__ void __launch_bounds__(kFarBlock) nearest_far_kernel(int n, const dou
                                                                 const float2* __restrict__ pf,
                                                                 const GridHead* __restrict__ h, double R,
                                                                 int* __restrict__ out) {
-  if (!h->use || !h->far) return;
+  if (!h->used() || !h->far) return;
   __shared__ int list[kFarBlock], listed;
   __shared__ double warp_d[kFarBlock / 32];
   __shared__ int warp_j[kFarBlock / 32];
@@ -816,13 +863,12 @@ GridHead* build_grid(int nq, const double* qx, const double* qy, int n, const do
   grid_box_kernel<<<blocks, 256, 0, st>>>(n, x, y, h);
   grid_size_kernel<<<1, 1, 0, st>>>(G, reach, h);
   grid_count_kernel<<<blocks, 256, 0, st>>>(n, x, y, G, h, *ends);
-  grid_scan_kernel<<<1, 1024, 0, st>>>(cells, h, *ends);
-  grid_fill_kernel<<<blocks, 256, 0, st>>>(n, x, y, G, h, *ends, *order);
   grid_work_kernel<<<std::min(blocks_of(nq, 256), 1216u), 256, 0, st>>>(nq, qx, qy, G, *ends, h);
-  grid_decide_kernel<<<1, 1, 0, st>>>((unsigned long long)nq * (unsigned long long)n, h);
+  grid_scan_kernel<<<1, 1024, 0, st>>>(cells, (unsigned long long)nq * (unsigned long long)n, h, *ends);
+  grid_fill_kernel<<<blocks, 256, 0, st>>>(n, x, y, G, h, *ends, *order);
   return h;
 }
-bool grid_worth(long long nq, long long n) { return n >= kGridMin && nq * n > kGridPairs; }
+bool grid_worth(long long nq, long long n, long long pairs) { return n >= kGridMin && nq * n > pairs; }
 
 // Lanes per query: the largest of `most`, most / 2, ... 1 whose grid still fits in
 // one wave of resident blocks (more lanes per query shorten each lane's scan;
@@ -938,7 +984,7 @@ void* points_ws(int n, void* ws, long long ws_bytes, bool* owned, cudaStream_t s
 // storage it takes, answered every query).
 void float2_copy(int n, const double* x, const double* y, float2* out, const GridHead* grid, cudaStream_t st) {
   const int blocks = (int)std::min<long long>(((long long)n + 255) / 256, 4096);
-  to_float2_kernel<<<blocks, 256, 0, st>>>(grid ? n - kHeadPoints : n, x, y, out, grid);
+  to_float2_kernel<<<blocks, 256, 0, st>>>(n, x, y, out, grid);
 }
 
 }  // namespace
@@ -961,13 +1007,17 @@ int hg_radius_best(int nq, const double* qx, const double* qy, int nr, const dou
   float2* rf = nr > 0 ? (float2*)points_ws(nr, workspace, workspace_bytes, &owned, st) : nullptr;
   if (nr > 0 && !rf) return HG_ERR_CUDA;
   GridHead* grid = nullptr;
-  if (grid_worth(nq, nr)) {
+  if (grid_worth(nq, nr, kRadiusPairs)) {
     int *ends, *order, G;
     // past the rounding of the query's own coordinate and of the pair test
     const double reach = eps * (1.0 + 0x1p-40) + 0x1p-40 * coord_max;
     grid = build_grid(nq, qx, qy, nr, rx, ry, reach, rf, &ends, &order, &G, st);
-    radius_grid_kernel<<<blocks_of(nq, 128), 128, 0, st>>>(nq, qx, qy, G, rx, ry, ends, order, grid, eps, reach,
-                                                                     coord_max, count, best_idx, best_d2);
+    auto kernel = radius_grid_kernel<1>;
+    const int S = lanes_per_query(radius_grid_kernel<4>, nq, 128, 4);
+    if (S == 2) kernel = radius_grid_kernel<2>;
+    if (S == 4) kernel = radius_grid_kernel<4>;
+    kernel<<<blocks_of((long long)nq * S, 128), 128, 0, st>>>(nq, qx, qy, G, rx, ry, ends, order, grid, eps, reach,
+                                                              coord_max, count, best_idx, best_d2);
   }
   if (nr > 0) float2_copy(nr, rx, ry, rf, grid, st);
   const int S = lanes_per_query(radius_best_kernel<8>, nq);
@@ -998,17 +1048,14 @@ int hg_nearest_neighbor(int n, const double* x, const double* y, double coord_ma
   float2* pf = (float2*)points_ws(n, workspace, workspace_bytes, &owned, st);
   if (!pf) return HG_ERR_CUDA;
   GridHead* grid = nullptr;
-  if (grid_worth(n, n)) {
+  if (grid_worth(n, n, kNearestPairs)) {
     int *ends, *order, G;
     grid = build_grid(n, x, y, n, x, y, 0.0, pf, &ends, &order, &G, st);
     const int S = lanes_per_query(nearest_grid_kernel<4>, n, 128, 4);
-    const unsigned blocks = blocks_of((long long)n * S, 128);
-    if (S == 4)
-      nearest_grid_kernel<4><<<blocks, 128, 0, st>>>(n, x, y, G, ends, order, grid, coord_max, out);
-    else if (S == 2)
-      nearest_grid_kernel<2><<<blocks, 128, 0, st>>>(n, x, y, G, ends, order, grid, coord_max, out);
-    else
-      nearest_grid_kernel<1><<<blocks, 128, 0, st>>>(n, x, y, G, ends, order, grid, coord_max, out);
+    auto kernel = nearest_grid_kernel<1>;
+    if (S == 2) kernel = nearest_grid_kernel<2>;
+    if (S == 4) kernel = nearest_grid_kernel<4>;
+    kernel<<<blocks_of((long long)n * S, 128), 128, 0, st>>>(n, x, y, G, ends, order, grid, coord_max, out);
   }
   float2_copy(n, x, y, pf, grid, st);
   if (grid) nearest_far_kernel<<<304, kFarBlock, 0, st>>>(n, x, y, pf, grid, coord_max, out);
