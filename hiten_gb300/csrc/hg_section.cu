@@ -350,9 +350,12 @@ __global__ void __launch_bounds__(kSecBlock) section_kernel(SecParams p) {
         left_hit = (gk1 <= 0.0) || (k - 1 >= 0 && g_prev >= 0.0);
       skip0 = left_hit;
     }
-    const unsigned cmask = __ballot_sync(0xFFFFFFFFu, cand);
-    if (cmask) {
+    if (__any_sync(0xFFFFFFFFu, cand)) {
       if (__any_sync(0xFFFFFFFFu, left_hit)) push(left_hit, k, -1);
+      // where one crossing is wanted, one at the segment's start is it, and the
+      // segment needs no scan (32 trajectories that start on the surface, 301
+      // samples, cubic: 92 -> 52 us)
+      const unsigned cmask = __ballot_sync(0xFFFFFFFFu, cand && !(left_hit && p.max_hits == 1));
       SegCtx c{gk, gk1, 0.0, 0.0, tk1 - tk, false};
       c.cub = p.cubic && c.dt > 0.0;
       if (cand && c.cub) {
