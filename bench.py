@@ -461,7 +461,7 @@ def bench_synodic_detect(args):
           {"states": n, "samples": m, "segment_refine": 50, "interp": "cubic", "max_hits": 8},
           mean_hits=hits, linear={"ms": res["linear"][0], "mean_hits": res["linear"][1]},
           roofline={"bound": "fp64", "bytes_read": sample_bytes, "achieved_gbs": sample_bytes / (ms * 1e-3) / 1e9,
-                    "source": "the cubic Hermite evaluations and refinements hold the FP64 pipe; the scanned "
+                    "source": "FP64 chains of the cubic Hermite evaluations and refinements, few warps an SM; the scanned "
                               "components are read once"})
 
 

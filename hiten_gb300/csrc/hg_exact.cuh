@@ -4,9 +4,9 @@
 // GB300's FP64 unit takes one lane operation per half clock and SM (a warp
 // instruction holds it 16 cycles, and a warp alone waits 64 cycles for each),
 // while the SM issues up to four FP32 / integer warp instructions per clock.
-// A correctly rounded FP64 square root is about ten FP64 instructions, a
-// reciprocal six and a quotient three more; here they take none.  The
-// significands are exact integers, the estimates FP32:
+// A correctly rounded FP64 square root is eight FP64 instructions, a reciprocal
+// five and a quotient three more (44 of a 6-dim right-hand side's 75 with two
+// roots, two reciprocals and six quotients); here they take none.  The significands are exact integers, the estimates FP32:
 //   * a 24-bit first estimate from the FP32 reciprocal (square root),
 //   * two corrections, each the integer remainder of the estimate so far
 //     (modulo 2^32 or 2^64: the remainders are small, so the low bits are all

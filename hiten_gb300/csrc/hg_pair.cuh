@@ -830,7 +830,7 @@ __device__ __forceinline__ bool pair_dop_run(const LT& L, const DopParams& p, Pa
 
 // Blocks of one or two pairs, laid out as fixed_rk_pair_kernel's.
 // Six blocks of one pair per SM: 168 registers a thread (the dense cache of an
-// STM column, built once or never per trajectory, spills 100 bytes) and 36.5 KB
+// STM column, built once or never per trajectory, spills 100 bytes) and 29.5 KB
 // of shared memory; at the 255 registers taken unasked four blocks fit, and
 // 4096 trajectories (5.4 groups per SM) took two rounds.
 static __global__ void __launch_bounds__(128, 3) dop853_pair_kernel(DopParams p) {

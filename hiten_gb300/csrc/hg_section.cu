@@ -18,7 +18,9 @@
 // bounds for the skip, the Hermite basis at the scan's points formed once per
 // warp, every point evaluated once and handed to its neighbour -- and the
 // chains of the refinements, which ran one lane at a time before they were
-// queued.  20011 trajectories x 300 segments, cubic: 4.94 -> 0.70 ms.
+// queued.  20011 trajectories x 300 segments, cubic: 4.94 -> 0.70 ms (47 % of the
+// FP64 unit on 3.9 warps an SM; calls of the same launch lie between 0.69 and
+// 0.99 ms, by where its blocks land).
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -177,7 +179,8 @@ __device__ __forceinline__ bool sub_crosses(double g_lo, double g_hi, int direct
 }
 
 // One warp a block: warps differ in their candidates, and a block of several
-// holds its place until the slowest is done (cubic, us, blocks of 128 / 64 / 32:
+// holds its place until the slowest is done (cubic, us, blocks of 128 / 64 / 32
+// in one process:
 // 500 x 301 samples 657 / 619 / 593, 20011 x 301 918 / 803 / 738, 65536 x 301
 // 1703 / 1412 / 1316).
 constexpr int kSecBlock = 32;
