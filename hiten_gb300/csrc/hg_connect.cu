@@ -57,7 +57,7 @@ __device__ __forceinline__ void load_tile(Tile& T, const float2* __restrict__ pf
 // The grid's numbers, in the last 256 bytes of the workspace's 8 n.  Where the
 // grid is not used the FP32 copy takes their place too (the all-pairs scans have
 // no registers to spare for points that it leaves out), so `use` is set by a
-// pattern no FP32 copy has: two NaNs that no conversion returns.
+// pattern no FP32 copy has: two signalling NaNs, which no conversion returns.
 constexpr int kHeadPoints = 32;
 constexpr unsigned long long kUse = 0x7FA5A5A57FA5A5A5ull;
 struct GridHead {

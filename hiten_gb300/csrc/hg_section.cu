@@ -19,8 +19,8 @@
 // warp, every point evaluated once and handed to its neighbour -- and the
 // chains of the refinements, which ran one lane at a time before they were
 // queued.  20011 trajectories x 300 segments, cubic: 4.94 -> 0.70 ms (47 % of the
-// FP64 unit on 3.9 warps an SM; calls of the same launch lie between 0.69 and
-// 0.99 ms, by where its blocks land).
+// FP64 unit on 3.9 warps an SM; the same launch takes 0.69 to 1.26 ms from process
+// to process, by where its blocks land).
 #include <cuda_runtime.h>
 #include <math.h>
 
