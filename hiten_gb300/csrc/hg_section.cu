@@ -14,7 +14,7 @@
 // queue in segment order, which is the reference's stable ordering, and are
 // deduplicated against the last accepted hit as they stream out.
 //
-// What bounds it: the FP64 unit, so what the scan does is kept small -- FP32
+// What bounds it: a warp's FP64 chains, so what the scan does is kept small -- FP32
 // bounds for the skip, the Hermite basis at the scan's points formed once per
 // warp, every point evaluated once and handed to its neighbour -- and the
 // chains of the refinements, which ran one lane at a time before they were
